@@ -28,6 +28,7 @@
 
 #include "gbntt_arith.cuh"
 #include "gbntt_internal.h"
+#include "gbntt_p31.cuh"
 #include "gbntt.h"
 
 namespace gbntt {
@@ -63,6 +64,10 @@ struct PrimeSet {
 static const PrimeSet kSet2 = {2, {4, 3, 0}};       // lazy normal-form q0 + p3
 static const PrimeSet kSet2m = {2, {0, 3, 0}};      // Montgomery q0 + p3
 static const PrimeSet kSet3 = {3, {0, 1, 2}};
+// The 31-bit primes (indices 5..7, gbntt_p31.cuh): every product of 32-bit
+// coefficients of up to 3 2^25 points, unless three 64-bit primes or lazy q0
+// are asked for. All three share their launches.
+static const PrimeSet kSet31 = {3, {5, 6, 7}};
 
 struct Engine {
     bool ready = false;
@@ -87,6 +92,12 @@ struct Engine {
     uint64_t r3c[5] = {};           // per prime: c = (om - om^2) / 2 in its multiply form
     uint64_t r3rho[5] = {};         // per prime: rho (order 3 2^30), plain
     int r3_min_log = 20;            // radix-3 for c products of 3 2^k points when c 2^k >= 2^r3_min_log
+    bool p31 = true;                // 31-bit prime set where it fits
+    ShoupWord *d_st31 = nullptr;    // its step tables: [prime][dir][kP31StepWords]
+    uint32_t *d_tw31 = nullptr;     // its two-level tables: [prime][dir][2^10 hi | 2^15 lo], Montgomery form
+    uint32_t *d_rho31 = nullptr;    // radix-3: [prime][3 2^10 hi | 2^15 lo]
+    ShoupWord r3c31[3] = {};        // (om - om^2) / 2 per prime
+    uint64_t rho31[3] = {};         // rho (order 3 2^25) per prime
     bool batch_split = true;        // uneven batch products split into chunk products
     int split_ratio_log = 3;        // ... when the longer operand is >= 2^this x the shorter
     uint64_t garner2[2] = {0, 0};   // two-prime Garner constants (p3 Montgomery multipliers)
@@ -217,6 +228,13 @@ static cudaError_t launch_build_ptw_any(int pi, uint64_t *t, const uint64_t *hi,
     }
 }
 
+constexpr size_t kTw31Words = ((size_t)1 << (kP31MaxLog - kTwBits)) + kTwSize;        // two-level table, one prime and direction
+constexpr size_t kRho31Words = (3 * ((size_t)1 << (kP31MaxLog - kTwBits))) + kTwSize;
+static const uint32_t *tw31(int k, int dir, int lo)
+{
+    return g.d_tw31 + ((size_t)k * 2 + dir) * kTw31Words + (lo ? (size_t)1 << (kP31MaxLog - kTwBits) : 0);
+}
+
 // The table of one strided pass, or nullptr (tables off, over the budget,
 // allocation failed, or a stream capture in progress: the pass then forms
 // its twiddles itself). A new table is built on st and st is synchronised
@@ -232,12 +250,13 @@ static const uint64_t *pass_table(int pi, int dir, int log_m, int log_s, int sca
     if (it != g_ptw.end()) return it->second;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return nullptr;
-    const size_t bytes = ((size_t)1 << log_m) * (pi == 3 ? 4 : 8);
+    const size_t bytes = ((size_t)1 << log_m) * (pi == 3 || pi >= 5 ? 4 : 8);
     if (g_ptw_bytes + bytes > g.ptw_budget) return nullptr;
     uint64_t *d = nullptr;
     if (cudaMalloc(&d, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    const uint64_t *hi, *lo;
-    if (pi == 3) {
+    const uint64_t *hi = nullptr, *lo = nullptr;
+    if (pi >= 5) {
+    } else if (pi == 3) {
         hi = (const uint64_t *)(g.d_tw3 + ((size_t)dir * 2 + 0) * kTwSize);
         lo = (const uint64_t *)(g.d_tw3 + ((size_t)dir * 2 + 1) * kTwSize);
     } else {
@@ -245,7 +264,9 @@ static const uint64_t *pass_table(int pi, int dir, int log_m, int log_s, int sca
         hi = tw_ptr(ts, dir, 0);
         lo = tw_ptr(ts, dir, 1);
     }
-    cudaError_t e = launch_build_ptw_any(pi, d, hi, lo, log_m, log_s, scaled ? 1 : 0, scale, st);
+    cudaError_t e = pi >= 5 ? launch_p31_build_table(pi - 5, (uint32_t *)d, tw31(pi - 5, dir, 0), tw31(pi - 5, dir, 1),
+                                                     log_m, log_s, scaled ? 1 : 0, (uint32_t)scale, st)
+                            : launch_build_ptw_any(pi, d, hi, lo, log_m, log_s, scaled ? 1 : 0, scale, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { cudaFree(d); cudaGetLastError(); return nullptr; }
     g_ptw[key] = d;
@@ -298,6 +319,23 @@ int plan_passes(int log_n, int *p)
     return 2;
 }
 
+// Pass plan of a 2^log_n-point transform of the 31-bit prime set: the
+// override, or the fastest of the plans gbntt_autotune times.
+static int p31_plan(int log_n, int *p)
+{
+    constexpr int kLo = 11;
+    static const signed char kTuned[kP31MaxLog + 1 - kLo][1 + kMaxPasses] = {
+        {2, 5, 6},    {2, 6, 6},    {2, 5, 8},    {2, 6, 8},     // 2^11 .. 2^14
+        {2, 7, 8},    {2, 8, 8},    {2, 9, 8},    {2, 9, 9},     // 2^15 .. 2^18
+        {3, 6, 6, 7}, {3, 6, 7, 7}, {3, 7, 7, 7}, {3, 7, 7, 8},  // 2^19 .. 2^22
+        {3, 7, 8, 8}, {3, 8, 8, 8}, {3, 9, 8, 8},                // 2^23 .. 2^25
+    };
+    if (log_n < kLo || g_plan_override[log_n][0] > 0) return plan_passes(log_n, p);
+    const signed char *t = kTuned[log_n - kLo];
+    for (int i = 0; i < t[0]; i++) p[i] = t[1 + i];
+    return t[0];
+}
+
 static int choose_log(size_t na, size_t nb)
 {
     const size_t need = na + nb - 1;
@@ -327,7 +365,8 @@ static size_t workspace_bytes(int max_log)
     const size_t spec = 6 * n * sizeof(uint64_t);
     const size_t tw = 4 * 2 * 2 * (size_t)kTwSize * sizeof(uint64_t) + 2 * 2 * (size_t)kTwSize * sizeof(uint32_t) +
                       4 * 2 * (size_t)kStep1Words * sizeof(uint64_t) + 2 * (size_t)kStep1Words * sizeof(uint32_t) +
-                      4 * (size_t)kTwSize * (2 * sizeof(uint64_t) + sizeof(uint32_t));   // radix-3 rho tables
+                      4 * (size_t)kTwSize * (2 * sizeof(uint64_t) + sizeof(uint32_t)) +   // radix-3 rho tables
+                      6 * (size_t)kP31StepWords * sizeof(ShoupWord) + (6 * kTw31Words + 3 * kRho31Words) * sizeof(uint32_t);
     const size_t ctl = (2 + status_words(n)) * sizeof(unsigned);
     const size_t io = (4 * n + 64) * sizeof(uint32_t);
     return spec + tw + ctl + io;
@@ -346,6 +385,9 @@ static void free_all()
     cudaFree(g.d_tw3);
     cudaFree(g.d_st1);
     cudaFree(g.d_st13);
+    cudaFree(g.d_st31);
+    cudaFree(g.d_tw31);
+    cudaFree(g.d_rho31);
     for (int i = 0; i < 5; i++) cudaFree(g.d_r3[i]);
     cudaFree(g.d_ctl);
     cudaFree(g.d_io);
@@ -362,6 +404,52 @@ static void free_all()
     if (g.stream) cudaStreamDestroy(g.stream);
     invalidate_wave_graphs();
     g = Engine();
+}
+
+// Tables of the 31-bit prime set.
+static cudaError_t init_p31()
+{
+    constexpr int kHi = 1 << (kP31MaxLog - kTwBits);
+    std::vector<ShoupWord> st(6 * (size_t)kP31StepWords, ShoupWord{0, 0});
+    std::vector<uint32_t> tw(6 * kTw31Words), rt(3 * kRho31Words);
+    for (int k = 0; k < 3; k++) {
+        const uint64_t p = kP31[k];
+        auto mont = [&](uint64_t x) { return (uint32_t)((x << 32) % p); };
+        const uint64_t w = p31_pow(kP31Gen[k], (p - 1) >> kP31MaxLog, p);
+        for (int dir = 0; dir < 2; dir++) {
+            const uint64_t wd = dir ? p31_pow(w, p - 2, p) : w, big = p31_pow(wd, kTwSize, p);
+            uint32_t *t = tw.data() + ((size_t)k * 2 + dir) * kTw31Words;
+            uint64_t x = 1;
+            for (int i = 0; i < kHi; i++) { t[i] = mont(x); x = x * big % p; }
+            x = 1;
+            for (int i = 0; i < kTwSize; i++) { t[kHi + i] = mont(x); x = x * wd % p; }
+            ShoupWord *s = st.data() + ((size_t)k * 2 + dir) * kP31StepWords;
+            for (int l = kMinLog; l <= kMaxPassLog; l++) {
+                const int L = 1 << l, A = 1 << ((l + 1) / 2), B = 1 << (l / 2);
+                const uint64_t wl = p31_pow(wd, 1ull << (kP31MaxLog - l), p);
+                for (int ka = 0; ka < A; ka++)
+                    for (int b = 0; b < B; b++)
+                        s[L - 32 + ka * B + b] = s[kStep1Words + L - 32 + b * A + ka] =
+                            shoup_word(p31_pow(wl, (uint64_t)ka * b, p), p);
+            }
+        }
+        const uint64_t rho = p31_pow(kP31Gen[k], (p - 1) / (3ull << kP31MaxLog), p), big = p31_pow(rho, kTwSize, p);
+        uint32_t *t = rt.data() + k * kRho31Words;
+        uint64_t x = 1;
+        for (int i = 0; i < 3 * kHi; i++) { t[i] = mont(x); x = x * big % p; }
+        x = 1;
+        for (int i = 0; i < kTwSize; i++) { t[3 * kHi + i] = mont(x); x = x * rho % p; }
+        const uint64_t om = p31_pow(rho, 1ull << kP31MaxLog, p), om2 = om * om % p;
+        g.rho31[k] = rho;
+        g.r3c31[k] = shoup_word((om + p - om2) % p * ((p + 1) / 2) % p, p);
+    }
+    cudaError_t e = cudaMalloc(&g.d_st31, st.size() * sizeof(ShoupWord));
+    if (e == cudaSuccess) e = cudaMalloc(&g.d_tw31, tw.size() * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&g.d_rho31, rt.size() * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemcpy(g.d_st31, st.data(), st.size() * sizeof(ShoupWord), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(g.d_tw31, tw.data(), tw.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(g.d_rho31, rt.data(), rt.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    return e;
 }
 
 static int init_impl(int max_log)
@@ -535,6 +623,13 @@ static int init_impl(int max_log)
         g.garner2[1] = (uint64_t)(((u128)1 << 64) % p);
     }
 
+    if (init_p31() != cudaSuccess) {
+        set_err("gbntt_init: tables of the 31-bit primes failed");
+        cudaGetLastError();
+        free_all();
+        return GBNTT_ERR_ALLOC;
+    }
+
     // Garner constants (Montgomery forms):
     //   [0] q0^-1 mod q1, [1] q0 mod q2, [2] (q0 q1)^-1 mod q2.
     const uint64_t q0 = prime_value(0), q1 = prime_value(1), q2 = prime_value(2);
@@ -556,6 +651,8 @@ static int init_impl(int max_log)
         // against 101 ms lazy at 2^28 limbs) and the two-stream overlap
         const char *qf = getenv("GBNTT_Q0_FORM");
         g.q0_lazy = qf && qf[0] == 'l';
+        const char *sp = getenv("GBNTT_P31");   // 0: q0 with p3 for every length
+        g.p31 = !g.q0_lazy && !(sp && sp[0] == '0');
         const char *ov = getenv("GBNTT_OVERLAP");
         g.overlap = !(ov && ov[0] == '0');
         // (measured at 2^28 limbs through ntt_bigint_mul: 105 ms against 110 ms
@@ -611,7 +708,17 @@ static TwTables tables(const PrimeSet &ps, int dir)
 }
 
 static const PrimeSet &coef32_set() { return g.prime_set == 3 ? kSet3 : (g.q0_lazy ? kSet2 : kSet2m); }
-static double word_bytes(int pi) { return pi == 3 ? 4.0 : 8.0; }
+static double word_bytes(int pi) { return pi == 3 || pi >= 5 ? 4.0 : 8.0; }
+
+// Whether transforms of 2^L points (or 3 2^L, r3) of 32-bit coefficients use
+// the 31-bit prime set: its roots of unity end at 2^25, and a limb-reading
+// first pass is a strided one (plans of two or more passes). The shorter
+// operand of such a product has at most 3 2^24 limbs, far below the 2^28
+// that the three primes carry.
+static bool use_p31(int L, bool r3)
+{
+    return g.p31 && g.prime_set == 2 && L <= kP31MaxLog && (r3 || L > kMaxPassLog);
+}
 
 // Overlap of the two-prime set: slot 1's passes go to an auxiliary stream
 // forked from st before the first forward pass and joined back before the
@@ -809,12 +916,199 @@ static int inner_fused(const PrimeSet &ps, uint64_t *specA, const uint64_t *spec
     return GBNTT_OK;
 }
 
+// ---- the pass chain of the 31-bit prime set ----
+
+// One operand of a chain: W transforms of 2^L points at spec + k stride
+// 64-bit words (prime k), read from limbs (one product) or limb_tab.
+struct P31Op {
+    uint64_t *spec;
+    long long W;
+    const uint32_t *limbs;
+    size_t n;
+    const uint32_t *const *limb_tab;
+    const long long *len_tab;
+};
+
+// Forward passes but the innermost one of nops operands (those of equal W in
+// one launch). preloaded: the spectra hold residues already.
+static int p31_forward(const P31Op *ops, int nops, size_t stride, int L, cudaStream_t st, bool preloaded)
+{
+    int pl[kMaxPasses];
+    const int np = p31_plan(L, pl);
+    const bool together = nops == 2 && ops[0].W == ops[1].W;
+    int log_m = L;
+    for (int i = 0; i + 1 < np; i++) {
+        P31PassArgs a;
+        memset(&a, 0, sizeof a);
+        a.log_m = log_m;
+        a.log_s = log_m - pl[i];
+        a.log_prod = L;
+        for (int k = 0; k < 3; k++) {
+            a.ptw[k] = (const uint32_t *)pass_table(5 + k, 0, a.log_m, a.log_s, 0, 0, st);
+            a.st[k] = g.d_st31 + ((size_t)k * 2 + 0) * kP31StepWords;
+            a.hi[k] = tw31(k, 0, 0);
+            a.lo[k] = tw31(k, 0, 1);
+        }
+        for (int o = 0; o < nops; o += together ? 2 : 1) {
+            const int n = together ? 2 : 1;
+            double bytes = 0;
+            for (int q = 0; q < n; q++) {
+                const P31Op &op = ops[o + q];
+                for (int k = 0; k < 3; k++) a.data[q][k] = (uint32_t *)(op.spec + k * stride);
+                a.limbs[q] = op.limbs;
+                a.n_limbs[q] = (long long)op.n;
+                a.limb_tab[q] = op.limb_tab;
+                a.len_tab[q] = op.len_tab;
+                bytes += 12.0 * (double)((size_t)1 << L) * (double)op.W * (i == 0 && !preloaded ? 1.0 : 2.0) +
+                         (i == 0 && !preloaded ? 4.0 * (double)op.n : 0.0);
+            }
+            a.ncols = ops[o].W << (L - pl[i]);
+            rec_begin(st, i == 0 ? 0 : 1, pl[i], bytes);
+            CK(launch_p31_pass(pl[i], 0, i == 0 && !preloaded, n, a, st));
+            rec_end(st);
+        }
+        log_m -= pl[i];
+    }
+    return GBNTT_OK;
+}
+
+// How the second spectra of a wave belong to its products.
+enum P31Right { P31_OWN, P31_SQUARE, P31_SHARED, P31_PAIRED };
+
+// The factor of the last inverse pass: (2^L)^-1, or (3 2^L)^-1, times 2^32
+// for the Montgomery pointwise product, in Montgomery form.
+static uint32_t p31_scale(int k, int L, bool r3)
+{
+    const uint64_t p = kP31[k], n = (((uint64_t)1 << L) % p) * (r3 ? 3 : 1) % p;
+    const uint64_t c = (p31_pow(n, p - 2, p) << 32) % p;
+    return (uint32_t)((c << 32) % p);
+}
+
+// Innermost passes with the pointwise product, in place in specA, for W
+// transforms of 2^L points (r3: sub-transforms of products of 3 2^L). Also
+// clears the carry control words ctl[0] and ctl[2 .. 2 + nzero).
+static int p31_inner(uint64_t *specA, uint64_t *specB, size_t stride, int L, long long W, P31Right right, bool r3,
+                     unsigned *ctl, long long nzero, cudaStream_t st)
+{
+    int pl[kMaxPasses];
+    const int np = p31_plan(L, pl), l = pl[np - 1];
+    P31InnerArgs a;
+    memset(&a, 0, sizeof a);
+    for (int k = 0; k < 3; k++) {
+        a.st[k] = g.d_st31 + ((size_t)k * 2 + 0) * kP31StepWords;
+        a.sti[k] = g.d_st31 + ((size_t)k * 2 + 1) * kP31StepWords;
+        a.scale[k] = p31_scale(k, L, r3);
+    }
+    a.log_prod = L;
+    if (right == P31_SHARED) {   // the one right operand is finished first, then read by every product
+        for (int k = 0; k < 3; k++) a.data[k] = (uint32_t *)(specB + k * stride);
+        a.ncols = (r3 ? 3LL : 1LL) << (L - l);
+        rec_begin(st, 1, l, 24.0 * (double)((size_t)1 << L));
+        CK(launch_p31_contig_fwd(l, a, st));
+        rec_end(st);
+        a.other_done = 1;
+    }
+    for (int k = 0; k < 3; k++) {
+        a.data[k] = (uint32_t *)(specA + k * stride);
+        a.other[k] = right == P31_SQUARE ? nullptr : (uint32_t *)(specB + k * stride);
+    }
+    a.ncols = W << (L - l);
+    a.use_scale = np == 1;
+    a.shared = right == P31_SHARED;
+    a.paired = right == P31_PAIRED;
+    a.r3 = r3;
+    a.zero = ctl;
+    a.nzero = nzero;
+    rec_begin(st, 5, l, (right == P31_SQUARE ? 24.0 : 36.0) * (double)((size_t)1 << L) * (double)W);
+    CK(launch_p31_inner(l, a, st));
+    rec_end(st);
+    return GBNTT_OK;
+}
+
+// The inverse passes after the innermost one.
+static int p31_inverse(uint64_t *spec, size_t stride, int L, long long W, bool r3, cudaStream_t st)
+{
+    int pl[kMaxPasses], log_ms[kMaxPasses];
+    const int np = p31_plan(L, pl);
+    for (int i = 0, m = L; i < np; i++) { log_ms[i] = m; m -= pl[i]; }
+    for (int i = np - 2; i >= 0; i--) {
+        P31PassArgs a;
+        memset(&a, 0, sizeof a);
+        a.log_m = log_ms[i];
+        a.log_s = log_ms[i] - pl[i];
+        a.ncols = W << (L - pl[i]);
+        a.use_scale = i == 0;
+        for (int k = 0; k < 3; k++) {
+            a.data[0][k] = (uint32_t *)(spec + k * stride);
+            a.st[k] = g.d_st31 + ((size_t)k * 2 + 1) * kP31StepWords;
+            a.hi[k] = tw31(k, 1, 0);
+            a.lo[k] = tw31(k, 1, 1);
+            a.scale[k] = p31_scale(k, L, r3);
+            a.ptw[k] = (const uint32_t *)pass_table(5 + k, 1, a.log_m, a.log_s, i == 0 ? (r3 ? 2 : 1) : 0, a.scale[k], st);
+        }
+        rec_begin(st, 3, pl[i], 24.0 * (double)((size_t)1 << L) * (double)W);
+        CK(launch_p31_pass(pl[i], 1, false, 1, a, st));
+        rec_end(st);
+    }
+    return GBNTT_OK;
+}
+
+// The outer radix-3 stage of one operand's W products.
+static int p31_radix3(const P31Op &op, size_t stride, int k3, bool inverse, cudaStream_t st)
+{
+    P31R3Args a;
+    memset(&a, 0, sizeof a);
+    a.M = 1LL << k3;
+    a.W = op.W;
+    a.shift = kP31MaxLog - k3;
+    const long long per_block = 256LL * kR3Unroll;
+    a.blocks = (int)((a.M + per_block - 1) / per_block);
+    a.limbs = op.limbs;
+    a.n_limbs = (long long)op.n;
+    a.limb_tab = op.limb_tab;
+    a.len_tab = op.len_tab;
+    const uint64_t order = 3ull << kP31MaxLog;
+    uint64_t e = ((256ull * a.blocks) << a.shift) % order;
+    if (inverse && e) e = order - e;
+    for (int k = 0; k < 3; k++) {
+        a.spec[k] = (uint32_t *)(op.spec + k * stride);
+        a.rho[k] = g.d_rho31 + k * kRho31Words;
+        a.c[k] = g.r3c31[k];
+        a.step[k] = shoup_word(p31_pow(g.rho31[k], e, kP31[k]), kP31[k]);
+    }
+    const double nbw = 36.0 * (double)a.M * (double)a.W;
+    rec_begin(st, inverse ? 7 : 6, 0, inverse ? 2.0 * nbw : nbw + 4.0 * (double)op.n);
+    CK(launch_p31_radix3(inverse, a, st));
+    rec_end(st);
+    return GBNTT_OK;
+}
+
+// Residues of W products a b in A's spectra, ready for the carry kernel:
+// transforms of 2^L points, or 3 2^L (r3).
+static int p31_products(const P31Op &A, const P31Op &B, size_t stride, int L, bool r3, P31Right right, unsigned *ctl,
+                        long long nzero, cudaStream_t st)
+{
+    const P31Op in[2] = {A, B};
+    const int nops = right == P31_SQUARE ? 1 : 2;
+    P31Op sub[2] = {A, B};
+    int rc = GBNTT_OK;
+    if (r3)
+        for (int o = 0; o < nops; o++) {
+            if ((rc = p31_radix3(in[o], stride, L, false, st)) != GBNTT_OK) return rc;
+            sub[o].W *= 3;
+        }
+    if ((rc = p31_forward(sub, nops, stride, L, st, r3)) != GBNTT_OK) return rc;
+    if ((rc = p31_inner(A.spec, B.spec, stride, L, sub[0].W, right, r3, ctl, nzero, st)) != GBNTT_OK) return rc;
+    if ((rc = p31_inverse(A.spec, stride, L, sub[0].W, r3, st)) != GBNTT_OK) return rc;
+    return r3 ? p31_radix3(in[0], stride, L, true, st) : GBNTT_OK;
+}
+
 // Garner constants and residue pointers of a prime set into c.
 static void carry_setup(CarryArgs &c, const PrimeSet &ps, const uint64_t *specA, size_t stride)
 {
     for (int k = 0; k < ps.n; k++) c.res[k] = specA + k * stride;
-    c.mixed = ps.n == 2 ? 1 : 0;
-    if (c.mixed) {
+    c.set = ps.pi[0] >= 5 ? CARRY_SET_31 : ps.n == 2 ? CARRY_SET_2 : CARRY_SET_3;
+    if (c.set == CARRY_SET_2) {
         c.garner[0] = g.garner2[0];
         c.garner[1] = g.garner2[1];
     } else {
@@ -835,9 +1129,11 @@ static int carry(const PrimeSet &ps, uint32_t *d_c, size_t n_out, const uint64_t
     c.ticket = g.d_ctl;
     c.error = g.d_ctl + 1;
     c.status = g.d_ctl + 2;
-    const long long nt = carry_tiles((long long)n_out);
-    CK(cudaMemsetAsync(g.d_ctl, 0, sizeof(unsigned), st));
-    CK(cudaMemsetAsync(g.d_ctl + 2, 0, (size_t)nt * sizeof(unsigned), st));
+    if (c.set != CARRY_SET_31) {   // (cleared by the fused innermost passes there)
+        const long long nt = carry_tiles((long long)n_out);
+        CK(cudaMemsetAsync(g.d_ctl, 0, sizeof(unsigned), st));
+        CK(cudaMemsetAsync(g.d_ctl + 2, 0, (size_t)nt * sizeof(unsigned), st));
+    }
     double rb = 0;
     for (int k = 0; k < ps.n; k++) rb += word_bytes(ps.pi[k]);
     rec_begin(st, 4, 0, rb * (double)((size_t)1 << L) + 4.0 * (double)n_out);
@@ -988,6 +1284,29 @@ static int r3_residues(const uint32_t *d_a, size_t na, const uint32_t *d_b, size
     return join_aux(st, aux);
 }
 
+// c = a b on the 31-bit prime set. stage_a, stage_b: operands in host
+// memory, copied first (the transform of the product sizes this set takes is
+// short next to the host link).
+static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint32_t *d_b, size_t nb, int L, bool r3,
+                       cudaStream_t st, const StageJob *stage_b, uint32_t *stage_a)
+{
+    const bool square = (d_a == d_b && na == nb);
+    if (stage_a) {
+        CK(launch_copy_words(stage_a, d_a, (long long)na, g.sms * 4, st));
+        d_a = stage_a;
+        if (square) d_b = stage_a;
+    }
+    if (stage_b && !square) {
+        if (stage_b->mapped) CK(launch_copy_words(stage_b->dst, stage_b->src, (long long)stage_b->n, g.sms * 4, st));
+        else CK(cudaMemcpyAsync(stage_b->dst, stage_b->src, stage_b->n * 4, cudaMemcpyHostToDevice, st));
+    }
+    const P31Op A{g.d_spec, 1, d_a, na, nullptr, nullptr}, B{g.d_spec + 3 * g.n_max, 1, d_b, nb, nullptr, nullptr};
+    const int rc = p31_products(A, B, g.n_max, L, r3, square ? P31_SQUARE : P31_OWN, g.d_ctl,
+                                carry_tiles((long long)(na + nb)), st);
+    if (rc) return rc;
+    return carry(kSet31, d_c, na + nb, g.d_spec, g.n_max, L, st, r3 ? 3LL << L : 0);
+}
+
 // stage_a (optional): HBM copy of A made by its first pass (see forward).
 // stage_b (optional): copy of B into d_b, run on the copy stream while A is
 // transformed.
@@ -1007,7 +1326,9 @@ static int mul_dev(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint32_t
         return GBNTT_ERR_SIZE;
     }
     const int k3 = r3_log(na, nb);
-    if (k3 >= g.r3_min_log) return mul_dev_r3(d_c, d_a, na, d_b, nb, k3, st, stage_b, stage_a);
+    const bool r3 = k3 >= g.r3_min_log;
+    if (use_p31(r3 ? k3 : L, r3)) return mul_dev_p31(d_c, d_a, na, d_b, nb, r3 ? k3 : L, r3, st, stage_b, stage_a);
+    if (r3) return mul_dev_r3(d_c, d_a, na, d_b, nb, k3, st, stage_b, stage_a);
     const bool square = (d_a == d_b && na == nb);
     uint64_t *specA = g.d_spec;
     uint64_t *specB = g.d_spec + 3 * g.n_max;
@@ -1189,10 +1510,17 @@ static int wave_launches(BatchCtx &x, uint64_t *dtab, long long W, int L, cudaSt
                          long long tiles, bool shared_b, bool pair_b, bool r3)
 {
     uint64_t *specA = x.spec, *specB = x.spec + 3 * x.cap;
-    const PrimeSet &ps = coef32_set();
+    const bool p31 = use_p31(L, r3);
+    const PrimeSet &ps = p31 ? kSet31 : coef32_set();
     cudaStream_t aux = fork_aux(ps, st, aux_stream);
     int rc = GBNTT_OK;
-    if (r3) {
+    if (p31) {
+        const P31Op A{specA, W, nullptr, 0, (const uint32_t *const *)dtab, (const long long *)(dtab + W)};
+        const P31Op B{specB, shared_b ? 1 : pair_b ? W / 2 : W, nullptr, 0, (const uint32_t *const *)(dtab + 2 * W),
+                      (const long long *)(dtab + 3 * W)};
+        rc = p31_products(A, B, x.cap, L, r3, shared_b ? P31_SHARED : pair_b ? P31_PAIRED : P31_OWN, x.ctl, tiles, st);
+        if (rc) return rc;
+    } else if (r3) {
         // products of length 3 2^L: each operand's radix-3 stage, then its
         // three sub-transforms as a batch of 3 W for the pass chain (a
         // shared right operand: one product's three; pairs: W / 2 products')
@@ -1248,8 +1576,10 @@ static int wave_launches(BatchCtx &x, uint64_t *dtab, long long W, int L, cudaSt
     c.nprod = (int)W;
     c.log_n_prod = L;
     c.radix3 = r3 ? 1 : 0;
-    CK(cudaMemsetAsync(x.ctl, 0, sizeof(unsigned), st));
-    CK(cudaMemsetAsync(x.ctl + 2, 0, (size_t)tiles * sizeof(unsigned), st));
+    if (!p31) {   // (cleared by the fused innermost passes there)
+        CK(cudaMemsetAsync(x.ctl, 0, sizeof(unsigned), st));
+        CK(cudaMemsetAsync(x.ctl + 2, 0, (size_t)tiles * sizeof(unsigned), st));
+    }
     double rb = 0;
     for (int k = 0; k < ps.n; k++) rb += word_bytes(ps.pi[k]);
     const double npt = (double)((r3 ? 3LL : 1LL) << L);

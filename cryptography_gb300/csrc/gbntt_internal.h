@@ -86,6 +86,10 @@ struct PassArgs {
     uint64_t w64_inv[64];
 };
 
+// Residue arrays of the carry kernel: three 64-bit primes; q0 (64-bit words)
+// and p3 (32-bit words); the three 31-bit primes (32-bit words).
+enum CarrySet { CARRY_SET_3 = 0, CARRY_SET_2 = 1, CARRY_SET_31 = 2 };
+
 struct CarryArgs {
     const uint64_t *res[3];     // inverse-transform output, natural order
     uint32_t *out;              // product limbs (32-bit coefficient mode)
@@ -106,7 +110,7 @@ struct CarryArgs {
     int nprod;
     int log_n_prod;
     int radix3;                 // batched mode: products of 3 2^log_n_prod coefficients
-    int mixed;                  // two-prime set: res[0] q0 (64-bit), res[1] p3 (32-bit words)
+    int set;                    // CarrySet of res[]
 };
 
 enum ErrorBits : unsigned int {

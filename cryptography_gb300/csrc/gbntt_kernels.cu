@@ -17,6 +17,7 @@
 #include "gbntt_arith.cuh"
 #include "gbntt_carry.cuh"
 #include "gbntt_internal.h"
+#include "gbntt_p31_garner.cuh"
 
 namespace gbntt {
 
@@ -223,18 +224,31 @@ __device__ __forceinline__ void garner2_vals(const CarryArgs &a, uint64_t r0, ui
     if ((long long)top >= a.n_coef) err |= ERR_GARNER_DIGIT;
 }
 
-template <bool MIXED>
+// The 31-bit prime set. A true coefficient is below n_coef 2^64: a larger top
+// word means corrupted residues.
+__device__ __forceinline__ void garner31_vals(const CarryArgs &a, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t &w0,
+                                              uint32_t &w1, uint32_t &w2, unsigned &err)
+{
+    garner31(r0, r1, r2, w0, w1, w2);
+    if ((long long)w2 >= a.n_coef) err |= ERR_GARNER_DIGIT;
+}
+
+template <int SET>
 __device__ __forceinline__ void garner_any(const CarryArgs &a, long long j, uint32_t &w0, uint32_t &w1, uint32_t &w2,
                                            unsigned &err)
 {
-    if (MIXED) garner_coef2(a, j, w0, w1, w2, err);
+    if (SET == CARRY_SET_31) {
+        const bool in = j >= 0 && j < a.n_coef;
+        garner31_vals(a, in ? ((const uint32_t *)a.res[0])[j] : 0u, in ? ((const uint32_t *)a.res[1])[j] : 0u,
+                      in ? ((const uint32_t *)a.res[2])[j] : 0u, w0, w1, w2, err);
+    } else if (SET == CARRY_SET_2) garner_coef2(a, j, w0, w1, w2, err);
     else garner_coef(a, j, w0, w1, w2, err);
 }
 
 #ifndef GBNTT_CARRY_MIN_BLOCKS
 #define GBNTT_CARRY_MIN_BLOCKS 6   // resident carry CTAs per SM the register budget targets (2^29: 5 -> 2.39 ms, 6 -> 2.21, 8 -> 2.34)
 #endif
-template <bool BATCH, bool MIXED>
+template <bool BATCH, int SET>
 __global__ void __launch_bounds__(kCarryThreads, GBNTT_CARRY_MIN_BLOCKS) garner_carry_kernel_t(CarryArgs a)
 {
     constexpr int T = kCarryThreads, K = kCarryPerThread, TILE = kCarryTile;
@@ -264,7 +278,9 @@ __global__ void __launch_bounds__(kCarryThreads, GBNTT_CARRY_MIN_BLOCKS) garner_
         const long long b = s_prod;
         const long long n_prod = (a.radix3 ? 3LL : 1LL) << a.log_n_prod;
         const long long off = b * n_prod;
-        if (MIXED) {
+        if (SET == CARRY_SET_31) {
+            for (int pi = 0; pi < 3; pi++) a.res[pi] = (const uint64_t *)((const uint32_t *)a.res[pi] + off);
+        } else if (SET == CARRY_SET_2) {
             a.res[0] += off;
             a.res[1] = (const uint64_t *)((const uint32_t *)a.res[1] + off);
         } else {
@@ -280,7 +296,26 @@ __global__ void __launch_bounds__(kCarryThreads, GBNTT_CARRY_MIN_BLOCKS) garner_
     unsigned err = 0;
 
     // phase 1: coefficients of positions base-2 .. base+TILE-1 (slot q+2)
-    if constexpr (MIXED) {
+    if constexpr (SET == CARRY_SET_31) {
+        const uint32_t *r0 = (const uint32_t *)a.res[0], *r1 = (const uint32_t *)a.res[1];
+        const uint32_t *r2 = (const uint32_t *)a.res[2];
+        uint32_t v[K][3];
+#pragma unroll
+        for (int r = 0; r < K; r++) {
+            const long long j = base + r * T + tid;
+            const bool in = j < a.n_coef;
+            v[r][0] = in ? __ldcs(r0 + j) : 0u;
+            v[r][1] = in ? __ldcs(r1 + j) : 0u;
+            v[r][2] = in ? __ldcs(r2 + j) : 0u;
+        }
+#pragma unroll
+        for (int r = 0; r < K; r++) {
+            const int q = r * T + tid;
+            uint32_t w0, w1, w2;
+            garner31_vals(a, v[r][0], v[r][1], v[r][2], w0, w1, w2, err);
+            W0[spad(q + 2)] = w0; W1[spad(q + 2)] = w1; W2[spad(q + 2)] = w2;
+        }
+    } else if constexpr (SET == CARRY_SET_2) {
         // all of this thread's residue loads first (beyond the transform:
         // zero), then the arithmetic
         const uint64_t *res0 = a.res[0];
@@ -306,13 +341,13 @@ __global__ void __launch_bounds__(kCarryThreads, GBNTT_CARRY_MIN_BLOCKS) garner_
         for (int r = 0; r < K; r++) {
             const int q = r * T + tid;
             uint32_t w0, w1, w2;
-            garner_any<MIXED>(a, base + q, w0, w1, w2, err);
+            garner_any<SET>(a, base + q, w0, w1, w2, err);
             W0[spad(q + 2)] = w0; W1[spad(q + 2)] = w1; W2[spad(q + 2)] = w2;
         }
     }
     if (tid < 2) {
         uint32_t w0, w1, w2;
-        garner_any<MIXED>(a, base - 2 + tid, w0, w1, w2, err);
+        garner_any<SET>(a, base - 2 + tid, w0, w1, w2, err);
         W0[spad(tid)] = w0; W1[spad(tid)] = w1; W2[spad(tid)] = w2;
     }
     __syncthreads();
@@ -535,11 +570,26 @@ static void carry_carveout()
     static bool done = false;
     if (done) return;
     done = true;
-    cudaFuncSetAttribute(garner_carry_kernel_t<false, true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(garner_carry_kernel_t<false, false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(garner_carry_kernel_t<true, true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(garner_carry_kernel_t<true, false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    auto ask = [](auto fn) { cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100); };
+    ask(garner_carry_kernel_t<false, CARRY_SET_2>);
+    ask(garner_carry_kernel_t<false, CARRY_SET_3>);
+    ask(garner_carry_kernel_t<false, CARRY_SET_31>);
+    ask(garner_carry_kernel_t<true, CARRY_SET_2>);
+    ask(garner_carry_kernel_t<true, CARRY_SET_3>);
+    ask(garner_carry_kernel_t<true, CARRY_SET_31>);
     (void)cudaGetLastError();
+}
+
+template <bool BATCH>
+static cudaError_t launch_carry_set(const CarryArgs &args, long long nt, cudaStream_t stream)
+{
+    const unsigned grid = (unsigned)nt;
+    switch (args.set) {
+    case CARRY_SET_2: garner_carry_kernel_t<BATCH, CARRY_SET_2><<<grid, kCarryThreads, 0, stream>>>(args); break;
+    case CARRY_SET_31: garner_carry_kernel_t<BATCH, CARRY_SET_31><<<grid, kCarryThreads, 0, stream>>>(args); break;
+    default: garner_carry_kernel_t<BATCH, CARRY_SET_3><<<grid, kCarryThreads, 0, stream>>>(args); break;
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t launch_garner_carry(const CarryArgs &args, cudaStream_t stream, long long *ntiles_out)
@@ -548,18 +598,14 @@ cudaError_t launch_garner_carry(const CarryArgs &args, cudaStream_t stream, long
     const long long nt = carry_tiles(args.n_out);
     if (ntiles_out) *ntiles_out = nt;
     if (nt == 0) return cudaSuccess;
-    if (args.mixed) garner_carry_kernel_t<false, true><<<(unsigned)nt, kCarryThreads, 0, stream>>>(args);
-    else garner_carry_kernel_t<false, false><<<(unsigned)nt, kCarryThreads, 0, stream>>>(args);
-    return cudaGetLastError();
+    return launch_carry_set<false>(args, nt, stream);
 }
 
 cudaError_t launch_garner_carry_batch(const CarryArgs &args, long long grid_tiles, cudaStream_t stream)
 {
     carry_carveout();
     if (grid_tiles <= 0) return cudaSuccess;
-    if (args.mixed) garner_carry_kernel_t<true, true><<<(unsigned)grid_tiles, kCarryThreads, 0, stream>>>(args);
-    else garner_carry_kernel_t<true, false><<<(unsigned)grid_tiles, kCarryThreads, 0, stream>>>(args);
-    return cudaGetLastError();
+    return launch_carry_set<true>(args, grid_tiles, stream);
 }
 
 }  // namespace gbntt
