@@ -96,6 +96,7 @@ struct Engine {
     ShoupWord *d_st31 = nullptr;    // its step tables: [prime][dir][kP31StepWords]
     uint32_t *d_tw31 = nullptr;     // its two-level tables: [prime][dir][2^10 hi | 2^15 lo], Montgomery form
     uint32_t *d_rho31 = nullptr;    // radix-3: [prime][3 2^10 hi | 2^15 lo]
+    uint32_t *d_blk31 = nullptr;    // block kernel: [prime][dir], 2^(L + 1) words per length from offset 2^(L + 1)
     ShoupWord r3c31[3] = {};        // (om - om^2) / 2 per prime
     uint64_t rho31[3] = {};         // rho (order 3 2^25) per prime
     bool batch_split = true;        // uneven batch products split into chunk products
@@ -167,7 +168,7 @@ void set_error_message(const char *msg) { snprintf(g_err, sizeof g_err, "%s", ms
 // for roofline reporting; off by default and never used in timed runs.
 struct LaunchRec {
     int kind;       // 0 fwd first pass, 1 fwd pass, 2 inv first pass, 3 inv pass, 4 garner+carry,
-                    // 5 fused innermost passes, 6 and 7 forward and inverse radix-3 stages
+                    // 5 fused innermost passes, 6 and 7 forward and inverse radix-3 stages, 8 whole products
     int log_l;
     double bytes;   // algorithmic bytes moved by this launch
     cudaEvent_t e0, e1;
@@ -229,6 +230,7 @@ static cudaError_t launch_build_ptw_any(int pi, uint64_t *t, const uint64_t *hi,
 }
 
 constexpr size_t kTw31Words = ((size_t)1 << (kP31MaxLog - kTwBits)) + kTwSize;        // two-level table, one prime and direction
+constexpr size_t kBlk31Words = (size_t)4 << kP31BlockLog;
 constexpr size_t kRho31Words = (3 * ((size_t)1 << (kP31MaxLog - kTwBits))) + kTwSize;
 static const uint32_t *tw31(int k, int dir, int lo)
 {
@@ -366,7 +368,7 @@ static size_t workspace_bytes(int max_log)
     const size_t tw = 4 * 2 * 2 * (size_t)kTwSize * sizeof(uint64_t) + 2 * 2 * (size_t)kTwSize * sizeof(uint32_t) +
                       4 * 2 * (size_t)kStep1Words * sizeof(uint64_t) + 2 * (size_t)kStep1Words * sizeof(uint32_t) +
                       4 * (size_t)kTwSize * (2 * sizeof(uint64_t) + sizeof(uint32_t)) +   // radix-3 rho tables
-                      6 * (size_t)kP31StepWords * sizeof(ShoupWord) + (6 * kTw31Words + 3 * kRho31Words) * sizeof(uint32_t);
+                      6 * (size_t)kP31StepWords * sizeof(ShoupWord) + (6 * kTw31Words + 3 * kRho31Words + 6 * kBlk31Words) * sizeof(uint32_t);
     const size_t ctl = (2 + status_words(n)) * sizeof(unsigned);
     const size_t io = (4 * n + 64) * sizeof(uint32_t);
     return spec + tw + ctl + io;
@@ -388,6 +390,7 @@ static void free_all()
     cudaFree(g.d_st31);
     cudaFree(g.d_tw31);
     cudaFree(g.d_rho31);
+    cudaFree(g.d_blk31);
     for (int i = 0; i < 5; i++) cudaFree(g.d_r3[i]);
     cudaFree(g.d_ctl);
     cudaFree(g.d_io);
@@ -411,7 +414,7 @@ static cudaError_t init_p31()
 {
     constexpr int kHi = 1 << (kP31MaxLog - kTwBits);
     std::vector<ShoupWord> st(6 * (size_t)kP31StepWords, ShoupWord{0, 0});
-    std::vector<uint32_t> tw(6 * kTw31Words), rt(3 * kRho31Words);
+    std::vector<uint32_t> tw(6 * kTw31Words), rt(3 * kRho31Words), blk(6 * kBlk31Words);
     for (int k = 0; k < 3; k++) {
         const uint64_t p = kP31[k];
         auto mont = [&](uint64_t x) { return (uint32_t)((x << 32) % p); };
@@ -423,6 +426,9 @@ static cudaError_t init_p31()
             for (int i = 0; i < kHi; i++) { t[i] = mont(x); x = x * big % p; }
             x = 1;
             for (int i = 0; i < kTwSize; i++) { t[kHi + i] = mont(x); x = x * wd % p; }
+            for (int l = kMinLog; l <= kP31BlockLog; l++)
+                p31_block_tables(l, blk.data() + ((size_t)k * 2 + dir) * kBlk31Words + ((size_t)2 << l),
+                                 p31_pow(wd, 1ull << (kP31MaxLog - l), p), p);
             ShoupWord *s = st.data() + ((size_t)k * 2 + dir) * kP31StepWords;
             for (int l = kMinLog; l <= kMaxPassLog; l++) {
                 const int L = 1 << l, A = 1 << ((l + 1) / 2), B = 1 << (l / 2);
@@ -446,6 +452,8 @@ static cudaError_t init_p31()
     cudaError_t e = cudaMalloc(&g.d_st31, st.size() * sizeof(ShoupWord));
     if (e == cudaSuccess) e = cudaMalloc(&g.d_tw31, tw.size() * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&g.d_rho31, rt.size() * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&g.d_blk31, blk.size() * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemcpy(g.d_blk31, blk.data(), blk.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(g.d_st31, st.data(), st.size() * sizeof(ShoupWord), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(g.d_tw31, tw.data(), tw.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(g.d_rho31, rt.data(), rt.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
@@ -710,15 +718,14 @@ static TwTables tables(const PrimeSet &ps, int dir)
 static const PrimeSet &coef32_set() { return g.prime_set == 3 ? kSet3 : (g.q0_lazy ? kSet2 : kSet2m); }
 static double word_bytes(int pi) { return pi == 3 || pi >= 5 ? 4.0 : 8.0; }
 
-// Whether transforms of 2^L points (or 3 2^L, r3) of 32-bit coefficients use
-// the 31-bit prime set: its roots of unity end at 2^25, and a limb-reading
-// first pass is a strided one (plans of two or more passes). The shorter
-// operand of such a product has at most 3 2^24 limbs, far below the 2^28
-// that the three primes carry.
-static bool use_p31(int L, bool r3)
-{
-    return g.p31 && g.prime_set == 2 && L <= kP31MaxLog && (r3 || L > kMaxPassLog);
-}
+// Whether transforms of 2^L points (or 3 2^L) of 32-bit coefficients use the
+// 31-bit prime set: its roots of unity end at 2^25. The shorter operand of
+// such a product has at most 3 2^24 limbs, far below the 2^28 that the three
+// primes carry.
+static bool use_p31(int L) { return g.p31 && g.prime_set == 2 && L <= kP31MaxLog; }
+
+// Whether a product of transform length 2^L runs in one CTA.
+static bool use_block(int L) { return use_p31(L) && L <= kP31BlockLog; }
 
 // Overlap of the two-prime set: slot 1's passes go to an auxiliary stream
 // forked from st before the first forward pass and joined back before the
@@ -1103,6 +1110,23 @@ static int p31_products(const P31Op &A, const P31Op &B, size_t stride, int L, bo
     return r3 ? p31_radix3(in[0], stride, L, true, st) : GBNTT_OK;
 }
 
+// W products of 2^L points, one CTA each (gbntt_p31_block.cu): the caller
+// fills in the operands.
+static int p31_block(P31BlockArgs &a, int L, long long W, unsigned *error, double bytes, cudaStream_t st)
+{
+    for (int k = 0; k < 3; k++) {
+        const uint64_t p = kP31[k];
+        for (int dir = 0; dir < 2; dir++)
+            a.tw[k][dir] = g.d_blk31 + ((size_t)k * 2 + dir) * kBlk31Words + ((size_t)2 << L);
+        a.scale[k] = shoup_word(((uint64_t)1 << (32 - L)) % p, p);
+    }
+    a.error = error;
+    rec_begin(st, 8, L, bytes);
+    CK(launch_p31_block(L, a, W, st));
+    rec_end(st);
+    return GBNTT_OK;
+}
+
 // Garner constants and residue pointers of a prime set into c.
 static void carry_setup(CarryArgs &c, const PrimeSet &ps, const uint64_t *specA, size_t stride)
 {
@@ -1300,6 +1324,17 @@ static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint
         if (stage_b->mapped) CK(launch_copy_words(stage_b->dst, stage_b->src, (long long)stage_b->n, g.sms * 4, st));
         else CK(cudaMemcpyAsync(stage_b->dst, stage_b->src, stage_b->n * 4, cudaMemcpyHostToDevice, st));
     }
+    if (!r3 && use_block(L)) {
+        P31BlockArgs a;
+        memset(&a, 0, sizeof a);
+        a.limbs[0] = d_a;
+        a.limbs[1] = d_b;
+        a.n_limbs[0] = (long long)na;
+        a.n_limbs[1] = (long long)nb;
+        a.out = d_c;
+        a.n_out = (long long)(na + nb);
+        return p31_block(a, L, 1, g.d_ctl + 1, 8.0 * (double)(na + nb), st);
+    }
     const P31Op A{g.d_spec, 1, d_a, na, nullptr, nullptr}, B{g.d_spec + 3 * g.n_max, 1, d_b, nb, nullptr, nullptr};
     const int rc = p31_products(A, B, g.n_max, L, r3, square ? P31_SQUARE : P31_OWN, g.d_ctl,
                                 carry_tiles((long long)(na + nb)), st);
@@ -1327,7 +1362,7 @@ static int mul_dev(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint32_t
     }
     const int k3 = r3_log(na, nb);
     const bool r3 = k3 >= g.r3_min_log;
-    if (use_p31(r3 ? k3 : L, r3)) return mul_dev_p31(d_c, d_a, na, d_b, nb, r3 ? k3 : L, r3, st, stage_b, stage_a);
+    if (use_p31(r3 ? k3 : L)) return mul_dev_p31(d_c, d_a, na, d_b, nb, r3 ? k3 : L, r3, st, stage_b, stage_a);
     if (r3) return mul_dev_r3(d_c, d_a, na, d_b, nb, k3, st, stage_b, stage_a);
     const bool square = (d_a == d_b && na == nb);
     uint64_t *specA = g.d_spec;
@@ -1499,7 +1534,8 @@ static int batch_wave(BatchCtx &x, const BatchItem *items, long long W, int L, c
     CK(cudaMemcpyAsync(dtab, h, (7 * (size_t)W + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     CK(cudaEventRecord(x.btab_ev[slot], st));
     *x.slot = slot ^ 1;
-    if (g.graphs && !g_rec_on) return wave_graph(x, dtab, W, L, st, aux_stream, tiles, shared_b, pair_b, r3);
+    // (a wave of one-CTA products is a single launch)
+    if (g.graphs && !g_rec_on && (r3 || !use_block(L))) return wave_graph(x, dtab, W, L, st, aux_stream, tiles, shared_b, pair_b, r3);
     return wave_launches(x, dtab, W, L, st, aux_stream, tiles, shared_b, pair_b, r3);
 }
 
@@ -1510,10 +1546,23 @@ static int wave_launches(BatchCtx &x, uint64_t *dtab, long long W, int L, cudaSt
                          long long tiles, bool shared_b, bool pair_b, bool r3)
 {
     uint64_t *specA = x.spec, *specB = x.spec + 3 * x.cap;
-    const bool p31 = use_p31(L, r3);
+    const bool p31 = use_p31(L);
     const PrimeSet &ps = p31 ? kSet31 : coef32_set();
     cudaStream_t aux = fork_aux(ps, st, aux_stream);
     int rc = GBNTT_OK;
+    if (!r3 && use_block(L)) {
+        P31BlockArgs a;
+        memset(&a, 0, sizeof a);
+        for (int o = 0; o < 2; o++) {
+            a.limb_tab[o] = (const uint32_t *const *)(dtab + 2 * o * W);
+            a.len_tab[o] = (const long long *)(dtab + (2 * o + 1) * W);
+        }
+        a.out_tab = (uint32_t *const *)(dtab + 4 * W);
+        a.nout_tab = (const long long *)(dtab + 5 * W);
+        a.shared = shared_b;
+        a.paired = pair_b;
+        return p31_block(a, L, W, x.ctl + 1, 16.0 * (double)((size_t)1 << L) * (double)W, st);
+    }
     if (p31) {
         const P31Op A{specA, W, nullptr, 0, (const uint32_t *const *)dtab, (const long long *)(dtab + W)};
         const P31Op B{specB, shared_b ? 1 : pair_b ? W / 2 : W, nullptr, 0, (const uint32_t *const *)(dtab + 2 * W),
@@ -1752,7 +1801,7 @@ static int batch_mul(uint32_t *const *d_c, const uint32_t *const *d_a, const siz
         const uint32_t *S = a_short ? d_a[i] : d_b[i], *Bp = a_short ? d_b[i] : d_a[i];
         int ls = kMinLog;
         while (((size_t)1 << ls) < 4 * nS) ls++;
-        if (g.batch_split && nS >= kSplitMinShort && L > ls && nB >= (nS << g.split_ratio_log)) {
+        if (g.batch_split && nS >= kSplitMinShort && L > ls && !use_block(L) && nB >= (nS << g.split_ratio_log)) {
             const size_t chunk = ((size_t)1 << ls) - nS + 1;
             const size_t n_out = nB + nS;
             void *E = nullptr, *O = nullptr;

@@ -299,6 +299,28 @@ struct P31R3Args {
 };
 cudaError_t launch_p31_radix3(bool inverse, const P31R3Args &a, cudaStream_t st);
 
+// A whole product of up to 2^kP31BlockLog coefficients in one CTA (W of them:
+// the tables, one CTA each).
+constexpr int kP31BlockLog = 12;
+struct P31BlockArgs {
+    const uint32_t *limbs[2];
+    long long n_limbs[2];
+    uint32_t *out;
+    long long n_out;
+    const uint32_t *const *limb_tab[2];
+    const long long *len_tab[2];
+    uint32_t *const *out_tab;
+    const long long *nout_tab;
+    int shared, paired;                 // second operands: entry 0 for all, entry b / 2
+    const uint32_t *tw[3][2];           // step tables per prime and direction (p31_block_tables)
+    ShoupWord scale[3];                 // 2^32 / N
+    unsigned *error;
+};
+cudaError_t launch_p31_block(int log_n, const P31BlockArgs &a, long long W, cudaStream_t st);
+// Fills the step tables of 2^log_n points for a root w of that order (at
+// most 2^(log_n + 1) words) and returns their size.
+int p31_block_tables(int log_n, uint32_t *dst, uint64_t w, uint64_t p);
+
 cudaError_t launch_p31_pass(int log_l, int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st);
 cudaError_t launch_p31_contig_fwd(int log_l, const P31InnerArgs &a, cudaStream_t st);
 cudaError_t launch_p31_inner(int log_l, const P31InnerArgs &a, cudaStream_t st);

@@ -82,6 +82,21 @@ def test_pass_sizes(engine, plan):
     assert engine.device_errors() == 0
 
 
+@pytest.mark.parametrize("L", range(5, 13))
+def test_one_cta_waves(engine, L):
+    # waves of products that run in one CTA each: own, paired and shared
+    # right operands, a square, one-limb operands
+    rng = np.random.default_rng(41 + L)
+    top = 1 << L
+    a, b, c = _rand(rng, top // 2), _rand(rng, top // 2 + 1), _rand(rng, 1)
+    d = _rand(rng, top - top // 3)
+    _waves(engine, [a, c, d, a], [b, d, c, a])
+    A = [a, a[1:], d[:top // 2], d[1:top // 2]]
+    _waves(engine, A, [b, b, a, a])
+    _waves(engine, A[1:], [b] * 3)
+    assert engine.device_errors() == 0
+
+
 def test_same_products_as_the_64bit_primes(engine):
     rng = np.random.default_rng(5)
     for na, nb in ((1, 1), (40, 3), (1500, 900), (70001, 333), (1 << 20, (1 << 20) + 1), (3 << 19, 3 << 19)):
