@@ -166,10 +166,8 @@ struct P31Shape {
     static constexpr int T = LOG_L == 5 ? 128 : 256;
     static constexpr int G = T / B;
     static constexpr int LOG_G = LOG_L == 5 ? 5 : 8 - LOG_B;
-    static constexpr int RS_S = B * G + (G < 32 ? G : 0);                      // strided: (ka, b, g) at ka RS_S + b G + g
     static constexpr int RS_C = B + 1;                                         // contiguous: g GS_C + ka RS_C + b
     static constexpr int GS_C = A * RS_C + (LOG_L == 5 ? 4 : LOG_L == 7 ? 8 : LOG_L == 9 ? 16 : 0);
-    static constexpr int WORDS_S = A * RS_S;
     static constexpr int WORDS_C = G * GS_C;
 };
 
@@ -177,27 +175,27 @@ struct P31Shape {
 // holds x[i] = element i B + b. Out: thread (g, q) holds element (q + r B) +
 // A kb in x[r B + kb]. st: step table w_L^(ka b) at [ka B + b]. Starts and
 // ends without a barrier; the buffer may be reused after one.
-template <int LOG_L, bool STRIDED>
+template <int LOG_L>
 __device__ __forceinline__ void p31_tile_fwd(uint32_t *x, uint32_t *sm, int g, int q, const ShoupWord *roots,
                                              const ShoupWord *__restrict__ st, uint32_t p)
 {
     using S = P31Shape<LOG_L>;
     constexpr int A = S::A, B = S::B;
     p31_dft<S::LOG_A>(x, roots, p);
-    uint32_t *w = STRIDED ? sm + q * S::G + g : sm + g * S::GS_C + q;
-    constexpr int RS = STRIDED ? S::RS_S : S::RS_C;
+    constexpr int RS = S::RS_C;
+    uint32_t *w = sm + g * S::GS_C + q;
 #pragma unroll
     for (int ka = 0; ka < A; ka++) {
         const uint32_t v = x[p31_bitrev(ka, S::LOG_A)];
         w[ka * RS] = ka == 0 ? v : p31_shoup(v, st[ka * B + q], p);
     }
     __syncthreads();
-    const uint32_t *r0 = STRIDED ? sm + q * RS + g : sm + g * S::GS_C + q * RS;
+    const uint32_t *r0 = sm + g * S::GS_C + q * RS;
 #pragma unroll
     for (int r = 0; r < S::R; r++) {
         uint32_t y[B];
 #pragma unroll
-        for (int b = 0; b < B; b++) y[b] = r0[r * B * RS + (STRIDED ? b * S::G : b)];
+        for (int b = 0; b < B; b++) y[b] = r0[r * B * RS + b];
         p31_dft<S::LOG_B>(y, roots, p);
 #pragma unroll
         for (int kb = 0; kb < B; kb++) x[r * B + kb] = y[p31_bitrev(kb, S::LOG_B)];
@@ -237,15 +235,6 @@ __device__ __forceinline__ void p31_tile_inv(uint32_t *x, uint32_t *sm, int g, i
     for (int i = 0; i < A; i++) x[i] = y[i];
 }
 
-// word at byte offset off of a base address
-__device__ __forceinline__ uint32_t ld_off(const void *base, uint32_t off)
-{
-    return *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(base) + off);
-}
-__device__ __forceinline__ void st_off(void *base, uint32_t off, uint32_t v)
-{
-    *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(base) + off) = v;
-}
 #endif  // __CUDACC__
 
 // Step tables of one prime and direction: for pass size 2^l the A x B block

@@ -61,10 +61,10 @@ p31_inner_kernel(const __grid_constant__ P31InnerArgs a)
     }
     const ShoupWord *st = a.st[k] + (L - 32), *sti = a.sti[k] + kStep1Words + (L - 32);
     const ShoupWord *wf = c_p31_roots.v[k][0], *wi = c_p31_roots.v[k][1];
-    p31_tile_fwd<LOG_L, false>(x, sm, g, q, wf, st, p);
+    p31_tile_fwd<LOG_L>(x, sm, g, q, wf, st, p);
     if (!SQUARE && !DONE) {
         __syncthreads();
-        p31_tile_fwd<LOG_L, false>(y, sm, g, q, wf, st, p);
+        p31_tile_fwd<LOG_L>(y, sm, g, q, wf, st, p);
     }
 #pragma unroll
     for (int i = 0; i < A; i++) x[i] = p31_mont(x[i], SQUARE ? x[i] : y[i], p, pinv);
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(P31Shape<LOG_L>::T) p31_contig_fwd_kernel(cons
     uint32_t x[A];
 #pragma unroll
     for (int i = 0; i < A; i++) x[i] = live ? d[i * B] : 0u;
-    p31_tile_fwd<LOG_L, false>(x, sm, g, q, c_p31_roots.v[k][0], a.st[k] + (L - 32), p);
+    p31_tile_fwd<LOG_L>(x, sm, g, q, c_p31_roots.v[k][0], a.st[k] + (L - 32), p);
     if (live) {
 #pragma unroll
         for (int r = 0; r < S::R; r++)

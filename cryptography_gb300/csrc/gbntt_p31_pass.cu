@@ -14,31 +14,95 @@ namespace gbntt {
 
 namespace {
 
+// Residues of one prime in a launch from which threads take two columns.
+// Measured per product, one column and two: 2^19 points 50.6 and 51.0 us (2^20
+// residues for both operands), 2^21 128 and 121 us, 2^23 447 and 410 us; at
+// 2^17 points the halved number of tiles costs more, 27.0 and 35.1 us.
+constexpr long long kTwoColumns = 1LL << 20;
+
+// word at byte offset off of a base address
+template <class Word>
+__device__ __forceinline__ Word ld_off(const void *base, uint32_t off)
+{
+    return *reinterpret_cast<const Word *>(reinterpret_cast<const char *>(base) + off);
+}
+template <class Word>
+__device__ __forceinline__ Word ldg_off(const void *base, uint32_t off)
+{
+    return __ldg(reinterpret_cast<const Word *>(reinterpret_cast<const char *>(base) + off));
+}
+template <class Word>
+__device__ __forceinline__ void st_off(void *base, uint32_t off, Word v)
+{
+    *reinterpret_cast<Word *>(reinterpret_cast<char *>(base) + off) = v;
+}
+
 // w^e (Montgomery form), e < 2^25, from the two-level tables
 __device__ __forceinline__ uint32_t p31_tw(const P31PassArgs &a, int k, uint32_t e, uint32_t p, uint32_t pinv)
 {
     return p31_mont(__ldg(a.hi[k] + (e >> 15)), __ldg(a.lo[k] + (e & 32767u)), p, pinv);
 }
 
-template <int LOG_L, int DIR, bool LIMBS>
-__global__ void __launch_bounds__(P31Shape<LOG_L>::T, LOG_L >= 9 ? 3 : LOG_L == 5 ? 10 : 5)
+// Shape of a strided tile with V adjacent columns per thread: GP threads
+// side by side, G = V GP columns. Exchange words are V residues wide, at
+// ka RS + b GP + gp.
+template <int LOG_L, int V, int DIR>
+struct P31StridedShape {
+    using S = P31Shape<LOG_L>;
+    static constexpr int B = S::B;
+    static constexpr int GP = V == 1 ? S::G : 16;
+    static constexpr int LOG_GP = GP == 8 ? 3 : GP == 16 ? 4 : 5;
+    static constexpr int G = V * GP;
+    static constexpr int T = GP * B;
+    static constexpr int LANES = 32 / V;   // threads served by one shared-memory access
+    static constexpr int RS = B * GP + (GP < LANES ? GP : 0);
+    static constexpr int MIN_BLOCKS = V == 1 ? (LOG_L >= 9 ? 3 : LOG_L == 5 ? 10 : 5)
+                                             : (LOG_L == 8 ? 3 + DIR : LOG_L == 5 ? 10 : 6);
+};
+template <int V>
+struct Residues;
+template <>
+struct Residues<1> {
+    typedef uint32_t T;
+    static __device__ __forceinline__ uint32_t get(uint32_t x, int) { return x; }
+    static __device__ __forceinline__ uint32_t make(const uint32_t *x, int) { return x[0]; }
+};
+template <>
+struct Residues<2> {
+    typedef uint2 T;
+    static __device__ __forceinline__ uint32_t get(uint2 x, int v) { return v ? x.y : x.x; }
+    static __device__ __forceinline__ uint2 make(const uint32_t *x, int n) { return make_uint2(x[0], x[n]); }
+};
+
+// One pass over V adjacent columns per thread. With two, the addresses, the
+// step twiddles' loads and the memory instructions are shared by two
+// residues: 42.5 instead of 50.9 instructions per residue of a 2^8-point
+// pass. A forward 2^8-point pass over 6 2^25 residues takes 317 us instead of
+// 352, an inverse one over half of them 156 instead of 180 (FMA-heavy pipe
+// 68%, issue 0.61, DRAM 51%). It wants twice the tiles to fill the GPU
+// (launch_l).
+template <int LOG_L, int DIR, bool LIMBS, int V>
+__global__ void __launch_bounds__(P31StridedShape<LOG_L, V, DIR>::T, P31StridedShape<LOG_L, V, DIR>::MIN_BLOCKS)
 p31_pass_kernel(const __grid_constant__ P31PassArgs a)
 {
     using S = P31Shape<LOG_L>;
-    constexpr int A = S::A, B = S::B, G = S::G;
-    __shared__ uint32_t sm[S::WORDS_S];
+    using H = P31StridedShape<LOG_L, V, DIR>;
+    using W = Residues<V>;
+    typedef typename W::T Word;
+    constexpr int A = S::A, B = S::B, GP = H::GP, RS = H::RS;
+    __shared__ Word sm[A * RS];
     const int k = blockIdx.x % 3, op = blockIdx.y;
-    const long long col0 = (long long)(blockIdx.x / 3) * G;
+    const long long col0 = (long long)(blockIdx.x / 3) * H::G;
     const uint32_t p = p31_prime(k), pinv = p31_inv(k);
-    const int t = threadIdx.x, g = t & (G - 1), q = t >> S::LOG_G;
+    const int t = threadIdx.x, gp = t & (GP - 1), q = t >> H::LOG_GP;
     const int log_s = a.log_s;
     const uint32_t sub0 = (uint32_t)((col0 >> log_s) << a.log_m);            // first element of the sub-problem
-    const uint32_t j = (uint32_t)(col0 & ((1LL << log_s) - 1)) + g;           // this thread's column
+    const uint32_t j = (uint32_t)(col0 & ((1LL << log_s) - 1)) + V * gp;      // this thread's (first) column
     uint32_t *data = a.data[op][k];
     // byte offsets: elements stay below 2^30 per prime
     const uint32_t step = (uint32_t)B << (log_s + 2);
     const uint32_t off0 = (sub0 + j + ((uint32_t)q << log_s)) << 2;
-    uint32_t x[A];
+    uint32_t x[V * A];   // column v's values at x[v A ..]
     if (LIMBS) {
         // the sub-problem is one product: its operand starts at sub0
         const uint32_t *limbs;
@@ -53,79 +117,142 @@ p31_pass_kernel(const __grid_constant__ P31PassArgs a)
         }
         const uint32_t nn = (uint32_t)n, r0 = j + ((uint32_t)q << log_s), rs = (uint32_t)B << log_s;
 #pragma unroll
-        for (int i = 0; i < A; i++) {
-            const uint32_t r = r0 + i * rs;
-            x[i] = r < nn ? __ldg(limbs + r) : 0u;
-        }
+        for (int i = 0; i < A; i++)
 #pragma unroll
-        for (int i = 0; i < A; i++) x[i] = p31_limb(x[i], p);
+            for (int v = 0; v < V; v++) {
+                const uint32_t r = r0 + i * rs + v;
+                x[v * A + i] = r < nn ? __ldg(limbs + r) : 0u;
+            }
+#pragma unroll
+        for (int i = 0; i < V * A; i++) x[i] = p31_limb(x[i], p);
     } else {
 #pragma unroll
-        for (int i = 0; i < A; i++) x[i] = ld_off(data, off0 + i * step);
+        for (int i = 0; i < A; i++) {
+            const Word w = ld_off<Word>(data, off0 + i * step);
+#pragma unroll
+            for (int v = 0; v < V; v++) x[v * A + i] = W::get(w, v);
+        }
     }
     const uint32_t *ptw = a.ptw[k];
     // table address such that an element's own offset indexes it
-    const char *tb = reinterpret_cast<const char *>(reinterpret_cast<uintptr_t>(ptw) - ((uintptr_t)sub0 << 2));
+    const void *tb = reinterpret_cast<const void *>(reinterpret_cast<uintptr_t>(ptw) - ((uintptr_t)sub0 << 2));
     if (DIR == 1) {
         if (ptw) {
-            uint32_t tw[A];
+            Word tw[A];
 #pragma unroll
-            for (int i = 0; i < A; i++) tw[i] = __ldg(reinterpret_cast<const uint32_t *>(tb + (off0 + i * step)));
+            for (int i = 0; i < A; i++) tw[i] = ldg_off<Word>(tb, off0 + i * step);
 #pragma unroll
-            for (int i = 0; i < A; i++) x[i] = p31_mont(x[i], tw[i], p, pinv);
+            for (int i = 0; i < A; i++)
+#pragma unroll
+                for (int v = 0; v < V; v++) x[v * A + i] = p31_mont(x[v * A + i], W::get(tw[i], v), p, pinv);
         } else {
             const int sh = kP31MaxLog - a.log_m;
             const uint32_t sc = a.scale[k];
 #pragma unroll
-            for (int i = 0; i < A; i++) {
-                uint32_t w = p31_tw(a, k, (uint32_t)(((uint64_t)(i * B + q) * j) << sh), p, pinv);
-                if (a.use_scale) w = p31_mont(w, sc, p, pinv);
-                x[i] = p31_mont(x[i], w, p, pinv);
-            }
+            for (int i = 0; i < A; i++)
+#pragma unroll
+                for (int v = 0; v < V; v++) {
+                    uint32_t w = p31_tw(a, k, (uint32_t)(((uint64_t)(i * B + q) * (j + v)) << sh), p, pinv);
+                    if (a.use_scale) w = p31_mont(w, sc, p, pinv);
+                    x[v * A + i] = p31_mont(x[v * A + i], w, p, pinv);
+                }
         }
     }
-    p31_tile_fwd<LOG_L, true>(x, sm, g, q, c_p31_roots.v[k][DIR], a.st[k] + (S::L - 32), p);
+    // step 1: DFTs over the high digit, step twiddles, exchange
+    const ShoupWord *roots = c_p31_roots.v[k][DIR], *__restrict__ st = a.st[k] + (S::L - 32);
+#pragma unroll
+    for (int v = 0; v < V; v++) p31_dft<S::LOG_A>(x + v * A, roots, p);
+    {
+        Word *w = sm + q * GP + gp;
+#pragma unroll
+        for (int ka = 0; ka < A; ka++) {
+            uint32_t y[V];
+            const int at = p31_bitrev(ka, S::LOG_A);
+            if (ka == 0) {
+#pragma unroll
+                for (int v = 0; v < V; v++) y[v] = x[v * A + at];
+            } else {
+                const ShoupWord f = st[ka * B + q];
+#pragma unroll
+                for (int v = 0; v < V; v++) y[v] = p31_shoup(x[v * A + at], f, p);
+            }
+            w[ka * RS] = W::make(y, 1);
+        }
+    }
+    __syncthreads();
+    // step 2: DFTs over the low digit, pass twiddles, store
     const uint32_t row = 4u << log_s;
-    if (DIR == 0) {
-        if (ptw) {
+    const Word *r0 = sm + q * RS + gp;
 #pragma unroll
-            for (int r = 0; r < S::R; r++) {
+    for (int r = 0; r < S::R; r++) {
+        uint32_t y[V * B];
 #pragma unroll
-                for (int kb = 0; kb < B; kb++) {
-                    const uint32_t off = off0 + (r * B + A * kb) * row;
-                    const uint32_t tw = __ldg(reinterpret_cast<const uint32_t *>(tb + off));
-                    st_off(data, off, p31_mont(x[r * B + kb], tw, p, pinv));
-                }
-            }
-        } else {
-            const int sh = kP31MaxLog - a.log_m;
+        for (int b = 0; b < B; b++) {
+            const Word w = r0[r * B * RS + b * GP];
 #pragma unroll
-            for (int r = 0; r < S::R; r++) {
-#pragma unroll
-                for (int kb = 0; kb < B; kb++) {
-                    const int m = q + r * B + A * kb;
-                    const uint32_t w = p31_tw(a, k, (uint32_t)(((uint64_t)m * j) << sh), p, pinv);
-                    st_off(data, off0 + (r * B + A * kb) * row, p31_mont(x[r * B + kb], w, p, pinv));
-                }
-            }
+            for (int v = 0; v < V; v++) y[v * B + b] = W::get(w, v);
         }
-    } else {
+        // twiddles in groups, a group's loads all in flight; with two columns the
+        // first group's are issued before the DFT
+        constexpr int C = V == 1 ? (B < 16 ? B : 16) : (B < 8 ? B : 8);
+        Word tw0[C];
+        if (V == 2 && DIR == 0 && ptw) {
 #pragma unroll
-        for (int r = 0; r < S::R; r++) {
+            for (int c = 0; c < C; c++) tw0[c] = ldg_off<Word>(tb, off0 + (r * B + A * c) * row);
+        }
 #pragma unroll
-            for (int kb = 0; kb < B; kb++) st_off(data, off0 + (r * B + A * kb) * row, x[r * B + kb]);
+        for (int v = 0; v < V; v++) p31_dft<S::LOG_B>(y + v * B, roots, p);
+#pragma unroll
+        for (int k0 = 0; k0 < B; k0 += C) {
+            Word tw[C];
+            if (DIR == 0 && ptw) {
+#pragma unroll
+                for (int c = 0; c < C; c++)
+                    tw[c] = V == 2 && k0 == 0 ? tw0[c] : ldg_off<Word>(tb, off0 + (r * B + A * (k0 + c)) * row);
+            }
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                const int kb = k0 + c;
+                uint32_t z[V];
+#pragma unroll
+                for (int v = 0; v < V; v++) z[v] = y[v * B + p31_bitrev(kb, S::LOG_B)];
+                if (DIR == 0) {
+                    if (ptw) {
+#pragma unroll
+                        for (int v = 0; v < V; v++) z[v] = p31_mont(z[v], W::get(tw[c], v), p, pinv);
+                    } else {
+                        const int sh = kP31MaxLog - a.log_m, m = q + r * B + A * kb;
+#pragma unroll
+                        for (int v = 0; v < V; v++)
+                            z[v] = p31_mont(z[v], p31_tw(a, k, (uint32_t)(((uint64_t)m * (j + v)) << sh), p, pinv), p, pinv);
+                    }
+                }
+                st_off<Word>(data, off0 + (r * B + A * kb) * row, W::make(z, 1));
+            }
         }
     }
+}
+
+template <int LOG_L, int V>
+void launch_v(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
+{
+    using H = P31StridedShape<LOG_L, V, 0>;
+    const dim3 grid((unsigned)(3 * (a.ncols / H::G)), (unsigned)nops);
+    if (dir == 1) p31_pass_kernel<LOG_L, 1, false, V><<<grid, H::T, 0, st>>>(a);
+    else if (limbs) p31_pass_kernel<LOG_L, 0, true, V><<<grid, H::T, 0, st>>>(a);
+    else p31_pass_kernel<LOG_L, 0, false, V><<<grid, H::T, 0, st>>>(a);
 }
 
 template <int LOG_L>
 cudaError_t launch_l(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
 {
-    using S = P31Shape<LOG_L>;
-    const dim3 grid((unsigned)(3 * (a.ncols / S::G)), (unsigned)nops);
-    if (dir == 1) p31_pass_kernel<LOG_L, 1, false><<<grid, S::T, 0, st>>>(a);
-    else if (limbs) p31_pass_kernel<LOG_L, 0, true><<<grid, S::T, 0, st>>>(a);
-    else p31_pass_kernel<LOG_L, 0, false><<<grid, S::T, 0, st>>>(a);
+    if constexpr (LOG_L <= 8) {   // (more points leave too few warps: 32 or more residues per column in registers)
+        if ((a.ncols << LOG_L) * nops >= kTwoColumns) {
+            launch_v<LOG_L, 2>(dir, limbs, nops, a, st);
+            return cudaGetLastError();
+        }
+    }
+    launch_v<LOG_L, 1>(dir, limbs, nops, a, st);
     return cudaGetLastError();
 }
 
