@@ -329,7 +329,7 @@ static int p31_plan(int log_n, int *p)
     static const signed char kTuned[kP31MaxLog + 1 - kLo][1 + kMaxPasses] = {
         {2, 5, 6},    {2, 6, 6},    {2, 7, 6},    {2, 6, 8},     // 2^11 .. 2^14
         {2, 7, 8},    {2, 8, 8},    {2, 9, 8},    {2, 9, 9},     // 2^15 .. 2^18
-        {2, 10, 9},   {2, 10, 10},  {3, 7, 7, 7}, {3, 7, 7, 8},  // 2^19 .. 2^22
+        {3, 5, 6, 8}, {3, 5, 7, 8}, {3, 7, 7, 7}, {3, 7, 7, 8},  // 2^19 .. 2^22
         {3, 8, 7, 8}, {3, 8, 8, 8}, {3, 9, 8, 8},                // 2^23 .. 2^25
     };
     if (log_n < kLo || g_plan_override[log_n][0] > 0) return plan_passes(log_n, p);

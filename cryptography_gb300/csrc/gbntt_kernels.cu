@@ -258,6 +258,7 @@ __global__ void __launch_bounds__(kCarryThreads, GBNTT_CARRY_MIN_BLOCKS) garner_
     __shared__ unsigned s_tile, s_cin;
     __shared__ long long s_prod;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (SET == CARRY_SET_31) chain_wait();
     if (tid == 0) {
         s_tile = atomicAdd(a.ticket, 1u);
         if (BATCH) {
@@ -586,7 +587,8 @@ static cudaError_t launch_carry_set(const CarryArgs &args, long long nt, cudaStr
     const unsigned grid = (unsigned)nt;
     switch (args.set) {
     case CARRY_SET_2: garner_carry_kernel_t<BATCH, CARRY_SET_2><<<grid, kCarryThreads, 0, stream>>>(args); break;
-    case CARRY_SET_31: garner_carry_kernel_t<BATCH, CARRY_SET_31><<<grid, kCarryThreads, 0, stream>>>(args); break;
+    case CARRY_SET_31:
+        return launch_chained(garner_carry_kernel_t<BATCH, CARRY_SET_31>, dim3(grid), kCarryThreads, 0, stream, args);
     default: garner_carry_kernel_t<BATCH, CARRY_SET_3><<<grid, kCarryThreads, 0, stream>>>(args); break;
     }
     return cudaGetLastError();

@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(BlockShape<LOG_N>::T) p31_block_kernel(const _
     uint32_t *out;
     long long n_out;
     const long long b = blockIdx.x;
+    chain_wait();
     if (a.limb_tab[0]) {
         const long long bb = a.shared ? 0 : a.paired ? b >> 1 : b;
         in[0] = a.limb_tab[0][b];
@@ -276,8 +277,7 @@ cudaError_t launch_n(const P31BlockArgs &a, long long W, cudaStream_t st)
         static const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
         if (e != cudaSuccess) return e;
     }
-    fn<<<(unsigned)W, S::T, S::SMEM, st>>>(a);
-    return cudaGetLastError();
+    return launch_chained(fn, dim3((unsigned)W), S::T, S::SMEM, st, a);
 }
 
 template <int LOG_N>

@@ -36,6 +36,7 @@ p31_inner_kernel(const __grid_constant__ P31InnerArgs a)
     const int t = threadIdx.x, q = t & (B - 1), g = t >> S::LOG_B;
     const bool live = col0 + g < a.ncols;
     const long long col = live ? col0 + g : 0;   // columns beyond the last one load zeros and store nothing
+    chain_wait();
     if (a.zero && k == 0) {
         const long long n = a.nzero, at = (long long)(blockIdx.x / 3) * S::T + t, by = (long long)(gridDim.x / 3) * S::T;
         if (at == 0) a.zero[0] = 0;
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(P31Shape<LOG_L>::T) p31_contig_fwd_kernel(cons
     const bool live = col0 + g < a.ncols;
     uint32_t *d = a.data[k] + ((live ? col0 + g : 0) << LOG_L) + q;
     uint32_t x[A];
+    chain_wait();
 #pragma unroll
     for (int i = 0; i < A; i++) x[i] = live ? d[i * B] : 0u;
     p31_tile_fwd<LOG_L>(x, sm, g, q, c_p31_roots.v[k][0], a.st[k] + (L - 32), p);
@@ -112,18 +114,17 @@ cudaError_t launch_inner_l(const P31InnerArgs &a, cudaStream_t st)
 {
     using S = P31Shape<LOG_L>;
     const unsigned grid = (unsigned)(3 * ((a.ncols + S::G - 1) / S::G));
-    if (!a.other[0]) p31_inner_kernel<LOG_L, true, false><<<grid, S::T, 0, st>>>(a);
-    else if (a.other_done) p31_inner_kernel<LOG_L, false, true><<<grid, S::T, 0, st>>>(a);
-    else p31_inner_kernel<LOG_L, false, false><<<grid, S::T, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_chained(!a.other[0]    ? p31_inner_kernel<LOG_L, true, false>
+                          : a.other_done ? p31_inner_kernel<LOG_L, false, true>
+                                         : p31_inner_kernel<LOG_L, false, false>,
+                          dim3(grid), S::T, 0, st, a);
 }
 
 template <int LOG_L>
 cudaError_t launch_contig_l(const P31InnerArgs &a, cudaStream_t st)
 {
     using S = P31Shape<LOG_L>;
-    p31_contig_fwd_kernel<LOG_L><<<(unsigned)(3 * ((a.ncols + S::G - 1) / S::G)), S::T, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_chained(p31_contig_fwd_kernel<LOG_L>, dim3((unsigned)(3 * ((a.ncols + S::G - 1) / S::G))), S::T, 0, st, a);
 }
 
 }  // namespace

@@ -103,6 +103,7 @@ p31_pass_kernel(const __grid_constant__ P31PassArgs a)
     const uint32_t step = (uint32_t)B << (log_s + 2);
     const uint32_t off0 = (sub0 + j + ((uint32_t)q << log_s)) << 2;
     uint32_t x[V * A];   // column v's values at x[v A ..]
+    chain_wait();
     if (LIMBS) {
         // the sub-problem is one product: its operand starts at sub0
         const uint32_t *limbs;
@@ -234,26 +235,23 @@ p31_pass_kernel(const __grid_constant__ P31PassArgs a)
 }
 
 template <int LOG_L, int V>
-void launch_v(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
+cudaError_t launch_v(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
 {
     using H = P31StridedShape<LOG_L, V, 0>;
     const dim3 grid((unsigned)(3 * (a.ncols / H::G)), (unsigned)nops);
-    if (dir == 1) p31_pass_kernel<LOG_L, 1, false, V><<<grid, H::T, 0, st>>>(a);
-    else if (limbs) p31_pass_kernel<LOG_L, 0, true, V><<<grid, H::T, 0, st>>>(a);
-    else p31_pass_kernel<LOG_L, 0, false, V><<<grid, H::T, 0, st>>>(a);
+    return launch_chained(dir == 1 ? p31_pass_kernel<LOG_L, 1, false, V>
+                          : limbs  ? p31_pass_kernel<LOG_L, 0, true, V>
+                                   : p31_pass_kernel<LOG_L, 0, false, V>,
+                          grid, H::T, 0, st, a);
 }
 
 template <int LOG_L>
 cudaError_t launch_l(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
 {
     if constexpr (LOG_L <= 8) {   // (more points leave too few warps: 32 or more residues per column in registers)
-        if ((a.ncols << LOG_L) * nops >= kTwoColumns) {
-            launch_v<LOG_L, 2>(dir, limbs, nops, a, st);
-            return cudaGetLastError();
-        }
+        if ((a.ncols << LOG_L) * nops >= kTwoColumns) return launch_v<LOG_L, 2>(dir, limbs, nops, a, st);
     }
-    launch_v<LOG_L, 1>(dir, limbs, nops, a, st);
-    return cudaGetLastError();
+    return launch_v<LOG_L, 1>(dir, limbs, nops, a, st);
 }
 
 __global__ void p31_table_kernel(int k, uint32_t *table, const uint32_t *hi, const uint32_t *lo, int log_m, int log_s,

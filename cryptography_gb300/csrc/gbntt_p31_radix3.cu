@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(256, 4) p31_radix3_fwd_kernel(const __grid_con
     const uint32_t p = p31_prime(k), pinv = p31_inv(k);
     const uint32_t M = (uint32_t)a.M, G = (gridDim.x / 3) * 256u;
     const long long w = blockIdx.y;
+    chain_wait();
     const uint32_t *x = a.limb_tab ? a.limb_tab[w] : a.limbs;
     const uint32_t n = (uint32_t)(a.len_tab ? a.len_tab[w] : a.n_limbs);
     uint32_t *out = a.spec[k] + w * 3 * a.M;
@@ -71,6 +72,7 @@ __global__ void __launch_bounds__(256, 4) p31_radix3_inv_kernel(const __grid_con
     if (j >= M) return;
     const uint32_t ex = j << a.shift;
     uint32_t w1 = rho_pow(a.rho[k], ex ? kOrder - ex : 0u, p, pinv);   // w^(-j)
+    chain_wait();
     for (; j < M; j += U * G) {
         uint32_t v[U][3];
 #pragma unroll
@@ -100,9 +102,7 @@ cudaError_t launch_p31_radix3(bool inverse, const P31R3Args &a, cudaStream_t st)
 {
     if (a.W < 1 || a.W > 65535 || a.blocks < 1) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)(3 * a.blocks), (unsigned)a.W);
-    if (inverse) p31_radix3_inv_kernel<<<grid, 256, 0, st>>>(a);
-    else p31_radix3_fwd_kernel<<<grid, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_chained(inverse ? p31_radix3_inv_kernel : p31_radix3_fwd_kernel, grid, 256, 0, st, a);
 }
 
 }  // namespace gbntt
