@@ -97,6 +97,7 @@ struct Engine {
     uint32_t *d_tw31 = nullptr;     // its two-level tables: [prime][dir][2^10 hi | 2^15 lo], Montgomery form
     uint32_t *d_rho31 = nullptr;    // radix-3: [prime][3 2^10 hi | 2^15 lo]
     uint32_t *d_blk31 = nullptr;    // block kernel: [prime][dir], 2^(L + 1) words per length from offset 2^(L + 1)
+    uint32_t *d_g31 = nullptr;      // outer stage: [prime][dir][2^10 hi | 2^15 lo] powers of g, Montgomery form
     ShoupWord r3c31[3] = {};        // (om - om^2) / 2 per prime
     uint64_t rho31[3] = {};         // rho (order 3 2^25) per prime
     bool batch_split = true;        // uneven batch products split into chunk products
@@ -168,7 +169,8 @@ void set_error_message(const char *msg) { snprintf(g_err, sizeof g_err, "%s", ms
 // for roofline reporting; off by default and never used in timed runs.
 struct LaunchRec {
     int kind;       // 0 fwd first pass, 1 fwd pass, 2 inv first pass, 3 inv pass, 4 garner+carry,
-                    // 5 fused innermost passes, 6 and 7 forward and inverse radix-3 stages, 8 whole products
+                    // 5 fused innermost passes, 6 and 7 forward and inverse radix-3 stages, 8 whole products,
+                    // 9 and 10 forward and inverse outer stages
     int log_l;
     double bytes;   // algorithmic bytes moved by this launch
     cudaEvent_t e0, e1;
@@ -368,7 +370,7 @@ static size_t workspace_bytes(int max_log)
     const size_t tw = 4 * 2 * 2 * (size_t)kTwSize * sizeof(uint64_t) + 2 * 2 * (size_t)kTwSize * sizeof(uint32_t) +
                       4 * 2 * (size_t)kStep1Words * sizeof(uint64_t) + 2 * (size_t)kStep1Words * sizeof(uint32_t) +
                       4 * (size_t)kTwSize * (2 * sizeof(uint64_t) + sizeof(uint32_t)) +   // radix-3 rho tables
-                      6 * (size_t)kP31StepWords * sizeof(ShoupWord) + (6 * kTw31Words + 3 * kRho31Words + 6 * kBlk31Words) * sizeof(uint32_t);
+                      6 * (size_t)kP31StepWords * sizeof(ShoupWord) + (12 * kTw31Words + 3 * kRho31Words + 6 * kBlk31Words) * sizeof(uint32_t);
     const size_t ctl = (2 + status_words(n)) * sizeof(unsigned);
     const size_t io = (4 * n + 64) * sizeof(uint32_t);
     return spec + tw + ctl + io;
@@ -391,6 +393,7 @@ static void free_all()
     cudaFree(g.d_tw31);
     cudaFree(g.d_rho31);
     cudaFree(g.d_blk31);
+    cudaFree(g.d_g31);
     for (int i = 0; i < 5; i++) cudaFree(g.d_r3[i]);
     cudaFree(g.d_ctl);
     cudaFree(g.d_io);
@@ -414,7 +417,7 @@ static cudaError_t init_p31()
 {
     constexpr int kHi = 1 << (kP31MaxLog - kTwBits);
     std::vector<ShoupWord> st(6 * (size_t)kP31StepWords, ShoupWord{0, 0});
-    std::vector<uint32_t> tw(6 * kTw31Words), rt(3 * kRho31Words), blk(6 * kBlk31Words);
+    std::vector<uint32_t> tw(6 * kTw31Words), rt(3 * kRho31Words), blk(6 * kBlk31Words), gt(6 * kTw31Words);
     for (int k = 0; k < 3; k++) {
         const uint64_t p = kP31[k];
         auto mont = [&](uint64_t x) { return (uint32_t)((x << 32) % p); };
@@ -426,6 +429,13 @@ static cudaError_t init_p31()
             for (int i = 0; i < kHi; i++) { t[i] = mont(x); x = x * big % p; }
             x = 1;
             for (int i = 0; i < kTwSize; i++) { t[kHi + i] = mont(x); x = x * wd % p; }
+            const uint64_t gd = dir ? p31_pow(p31_outer_root(k), p - 2, p) : p31_outer_root(k);
+            const uint64_t gbig = p31_pow(gd, kTwSize, p);
+            t = gt.data() + ((size_t)k * 2 + dir) * kTw31Words;
+            x = 1;
+            for (int i = 0; i < kHi; i++) { t[i] = mont(x); x = x * gbig % p; }
+            x = 1;
+            for (int i = 0; i < kTwSize; i++) { t[kHi + i] = mont(x); x = x * gd % p; }
             for (int l = kMinLog; l <= kP31BlockLog; l++)
                 p31_block_tables(l, blk.data() + ((size_t)k * 2 + dir) * kBlk31Words + ((size_t)2 << l),
                                  p31_pow(wd, 1ull << (kP31MaxLog - l), p), p);
@@ -452,6 +462,9 @@ static cudaError_t init_p31()
     cudaError_t e = cudaMalloc(&g.d_st31, st.size() * sizeof(ShoupWord));
     if (e == cudaSuccess) e = cudaMalloc(&g.d_tw31, tw.size() * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&g.d_rho31, rt.size() * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&g.d_g31, gt.size() * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemcpy(g.d_g31, gt.data(), gt.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = p31_outer_init();
     if (e == cudaSuccess) e = cudaMalloc(&g.d_blk31, blk.size() * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemcpy(g.d_blk31, blk.data(), blk.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(g.d_st31, st.data(), st.size() * sizeof(ShoupWord), cudaMemcpyHostToDevice);
@@ -723,6 +736,18 @@ static double word_bytes(int pi) { return pi == 3 || pi >= 5 ? 4.0 : 8.0; }
 // such a product has at most 3 2^24 limbs, far below the 2^28 that the three
 // primes carry.
 static bool use_p31(int L) { return g.p31 && g.prime_set == 2 && L <= kP31MaxLog; }
+
+// Number of 2^25-point transforms of a product of more than 2^25
+// coefficients on the 31-bit prime set (gbntt_p31_outer.cu), 0 if it does not
+// take it: up to 2^29 coefficients and 2^28 limbs in the shorter operand,
+// whose coefficients are below 2^92.
+static int p31_outer_blocks(size_t na, size_t nb)
+{
+    const size_t need = na + nb - 1, blocks = (need + ((size_t)1 << kP31MaxLog) - 1) >> kP31MaxLog;
+    const bool fits = blocks > 1 && blocks <= (size_t)kP31MaxOuter &&
+                      std::min(na, nb) <= (size_t)1 << 28 && (blocks << kP31MaxLog) <= g.n_max;
+    return g.p31 && g.prime_set == 2 && fits ? (int)blocks : 0;
+}
 
 // Whether a product of transform length 2^L runs in one CTA.
 static bool use_block(int L) { return use_p31(L) && L <= kP31BlockLog; }
@@ -1090,24 +1115,55 @@ static int p31_radix3(const P31Op &op, size_t stride, int k3, bool inverse, cuda
     return GBNTT_OK;
 }
 
+// The outer stage of one product of up to R 2^25 coefficients.
+static int p31_outer(const P31Op &op, size_t stride, int R, bool inverse, cudaStream_t st)
+{
+    P31OuterArgs a;
+    memset(&a, 0, sizeof a);
+    a.limbs = op.limbs;
+    a.n_limbs = (long long)op.n;
+    a.blocks = (int)((op.n + ((size_t)1 << kP31MaxLog) - 1) >> kP31MaxLog);
+    for (int k = 0; k < 3; k++) {
+        a.spec[k] = (uint32_t *)(op.spec + k * stride);
+        a.g[k] = g.d_g31 + ((size_t)k * 2 + (inverse ? 1 : 0)) * kTw31Words;
+    }
+    const double nbw = 12.0 * (double)R * (double)((size_t)1 << kP31MaxLog);
+    rec_begin(st, inverse ? 10 : 9, R, inverse ? 2.0 * nbw : nbw + 4.0 * (double)op.n);
+    CK(launch_p31_outer(R, inverse, a, st));
+    rec_end(st);
+    return GBNTT_OK;
+}
+
 // Residues of W products a b in A's spectra, ready for the carry kernel:
-// transforms of 2^L points, or 3 2^L (r3).
-static int p31_products(const P31Op &A, const P31Op &B, size_t stride, int L, bool r3, P31Right right, unsigned *ctl,
-                        long long nzero, cudaStream_t st)
+// transforms of R 2^L points, R = 1, 3 (the radix-3 stage) or, with W = 1
+// and L = 25, up to kP31MaxOuter (the outer stage). b_ready (optional): an
+// event that B's limbs wait for; A is transformed first then.
+static int p31_products(const P31Op &A, const P31Op &B, size_t stride, int L, int R, P31Right right, unsigned *ctl,
+                        long long nzero, cudaStream_t st, cudaEvent_t b_ready = nullptr)
 {
     const P31Op in[2] = {A, B};
     const int nops = right == P31_SQUARE ? 1 : 2;
     P31Op sub[2] = {A, B};
     int rc = GBNTT_OK;
-    if (r3)
-        for (int o = 0; o < nops; o++) {
-            if ((rc = p31_radix3(in[o], stride, L, false, st)) != GBNTT_OK) return rc;
-            sub[o].W *= 3;
+    auto stage = [&](int o, bool inverse) {
+        return R == 3 ? p31_radix3(in[o], stride, L, inverse, st) : p31_outer(in[o], stride, R, inverse, st);
+    };
+    for (int o = 0; o < nops; o++) sub[o].W *= R;
+    if (b_ready && nops == 2) {
+        for (int o = 0; o < 2; o++) {
+            if (o == 1) CK(cudaStreamWaitEvent(st, b_ready, 0));
+            if (R > 1 && (rc = stage(o, false)) != GBNTT_OK) return rc;
+            if ((rc = p31_forward(sub + o, 1, stride, L, st, R > 1)) != GBNTT_OK) return rc;
         }
-    if ((rc = p31_forward(sub, nops, stride, L, st, r3)) != GBNTT_OK) return rc;
+    } else {
+        for (int o = 0; R > 1 && o < nops; o++)
+            if ((rc = stage(o, false)) != GBNTT_OK) return rc;
+        if ((rc = p31_forward(sub, nops, stride, L, st, R > 1)) != GBNTT_OK) return rc;
+    }
+    const bool r3 = R == 3;
     if ((rc = p31_inner(A.spec, B.spec, stride, L, sub[0].W, right, r3, ctl, nzero, st)) != GBNTT_OK) return rc;
     if ((rc = p31_inverse(A.spec, stride, L, sub[0].W, r3, st)) != GBNTT_OK) return rc;
-    return r3 ? p31_radix3(in[0], stride, L, true, st) : GBNTT_OK;
+    return R > 1 ? stage(0, true) : GBNTT_OK;
 }
 
 // W products of 2^L points, one CTA each (gbntt_p31_block.cu): the caller
@@ -1141,14 +1197,16 @@ static void carry_setup(CarryArgs &c, const PrimeSet &ps, const uint64_t *specA,
 }
 
 static int carry(const PrimeSet &ps, uint32_t *d_c, size_t n_out, const uint64_t *specA, size_t stride, int L,
-                 cudaStream_t st, long long n_coef = 0)
+                 cudaStream_t st, long long n_coef = 0, long long limit = 0)
 {
-    // n_coef: coefficients of the transform (2^L unless given: 3 2^k)
+    // n_coef: coefficients of the transform (2^L unless given); limit: no
+    // true coefficient reaches limit 2^64 (n_coef unless given)
     CarryArgs c;
     memset(&c, 0, sizeof c);
     carry_setup(c, ps, specA, stride);
     c.out = d_c;
     c.n_coef = n_coef ? n_coef : (long long)1 << L;
+    c.limit = limit ? limit : c.n_coef;
     c.n_out = (long long)n_out;
     c.ticket = g.d_ctl;
     c.error = g.d_ctl + 1;
@@ -1160,7 +1218,7 @@ static int carry(const PrimeSet &ps, uint32_t *d_c, size_t n_out, const uint64_t
     }
     double rb = 0;
     for (int k = 0; k < ps.n; k++) rb += word_bytes(ps.pi[k]);
-    rec_begin(st, 4, 0, rb * (double)((size_t)1 << L) + 4.0 * (double)n_out);
+    rec_begin(st, 4, 0, rb * (double)c.n_coef + 4.0 * (double)n_out);
     CK(launch_garner_carry(c, st, nullptr));
     rec_end(st);
     return GBNTT_OK;
@@ -1308,10 +1366,10 @@ static int r3_residues(const uint32_t *d_a, size_t na, const uint32_t *d_b, size
     return join_aux(st, aux);
 }
 
-// c = a b on the 31-bit prime set. stage_a, stage_b: operands in host
-// memory, copied first (the transform of the product sizes this set takes is
-// short next to the host link).
-static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint32_t *d_b, size_t nb, int L, bool r3,
+// c = a b on the 31-bit prime set, transforms of R 2^L points. stage_a,
+// stage_b: operands in host memory, copied first; with the outer stage the
+// copy of B runs while A is transformed.
+static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint32_t *d_b, size_t nb, int L, int R,
                        cudaStream_t st, const StageJob *stage_b, uint32_t *stage_a)
 {
     const bool square = (d_a == d_b && na == nb);
@@ -1320,11 +1378,23 @@ static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint
         d_a = stage_a;
         if (square) d_b = stage_a;
     }
+    cudaEvent_t b_ready = nullptr;
     if (stage_b && !square) {
-        if (stage_b->mapped) CK(launch_copy_words(stage_b->dst, stage_b->src, (long long)stage_b->n, g.sms * 4, st));
-        else CK(cudaMemcpyAsync(stage_b->dst, stage_b->src, stage_b->n * 4, cudaMemcpyHostToDevice, st));
+        cudaStream_t cs = st;
+        if (L == kP31MaxLog && R > 1) {   // after A's copy, which shares the host link
+            CK(cudaEventRecord(g.ev_a, st));
+            CK(cudaStreamWaitEvent(g.cstream, g.ev_a, 0));
+            cs = g.cstream;
+        }
+        if (stage_b->mapped)
+            CK(launch_copy_words(stage_b->dst, stage_b->src, (long long)stage_b->n, cs == st ? g.sms * 4 : g.sms / 2, cs));
+        else CK(cudaMemcpyAsync(stage_b->dst, stage_b->src, stage_b->n * 4, cudaMemcpyHostToDevice, cs));
+        if (cs != st) {
+            CK(cudaEventRecord(g.ev_b, cs));
+            b_ready = g.ev_b;
+        }
     }
-    if (!r3 && use_block(L)) {
+    if (R == 1 && use_block(L)) {
         P31BlockArgs a;
         memset(&a, 0, sizeof a);
         a.limbs[0] = d_a;
@@ -1336,10 +1406,10 @@ static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint
         return p31_block(a, L, 1, g.d_ctl + 1, 8.0 * (double)(na + nb), st);
     }
     const P31Op A{g.d_spec, 1, d_a, na, nullptr, nullptr}, B{g.d_spec + 3 * g.n_max, 1, d_b, nb, nullptr, nullptr};
-    const int rc = p31_products(A, B, g.n_max, L, r3, square ? P31_SQUARE : P31_OWN, g.d_ctl,
-                                carry_tiles((long long)(na + nb)), st);
+    const int rc = p31_products(A, B, g.n_max, L, R, square ? P31_SQUARE : P31_OWN, g.d_ctl,
+                                carry_tiles((long long)(na + nb)), st, b_ready);
     if (rc) return rc;
-    return carry(kSet31, d_c, na + nb, g.d_spec, g.n_max, L, st, r3 ? 3LL << L : 0);
+    return carry(kSet31, d_c, na + nb, g.d_spec, g.n_max, L, st, (long long)R << L, (long long)std::min(na, nb));
 }
 
 // stage_a (optional): HBM copy of A made by its first pass (see forward).
@@ -1362,7 +1432,9 @@ static int mul_dev(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint32_t
     }
     const int k3 = r3_log(na, nb);
     const bool r3 = k3 >= g.r3_min_log;
-    if (use_p31(r3 ? k3 : L)) return mul_dev_p31(d_c, d_a, na, d_b, nb, r3 ? k3 : L, r3, st, stage_b, stage_a);
+    if (use_p31(r3 ? k3 : L)) return mul_dev_p31(d_c, d_a, na, d_b, nb, r3 ? k3 : L, r3 ? 3 : 1, st, stage_b, stage_a);
+    if (const int R = p31_outer_blocks(na, nb))
+        return mul_dev_p31(d_c, d_a, na, d_b, nb, kP31MaxLog, R, st, stage_b, stage_a);
     if (r3) return mul_dev_r3(d_c, d_a, na, d_b, nb, k3, st, stage_b, stage_a);
     const bool square = (d_a == d_b && na == nb);
     uint64_t *specA = g.d_spec;
@@ -1567,7 +1639,7 @@ static int wave_launches(BatchCtx &x, uint64_t *dtab, long long W, int L, cudaSt
         const P31Op A{specA, W, nullptr, 0, (const uint32_t *const *)dtab, (const long long *)(dtab + W)};
         const P31Op B{specB, shared_b ? 1 : pair_b ? W / 2 : W, nullptr, 0, (const uint32_t *const *)(dtab + 2 * W),
                       (const long long *)(dtab + 3 * W)};
-        rc = p31_products(A, B, x.cap, L, r3, shared_b ? P31_SHARED : pair_b ? P31_PAIRED : P31_OWN, x.ctl, tiles, st);
+        rc = p31_products(A, B, x.cap, L, r3 ? 3 : 1, shared_b ? P31_SHARED : pair_b ? P31_PAIRED : P31_OWN, x.ctl, tiles, st);
         if (rc) return rc;
     } else if (r3) {
         // products of length 3 2^L: each operand's radix-3 stage, then its

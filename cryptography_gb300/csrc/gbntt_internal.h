@@ -95,6 +95,7 @@ struct CarryArgs {
     uint32_t *out;              // product limbs (32-bit coefficient mode)
     uint64_t *out64;            // product limbs (64-bit coefficient mode)
     long long n_coef;           // length of res[] (the transform length N)
+    long long limit;            // 31-bit primes: a true coefficient is below limit 2^64 (0: n_coef)
     long long n_out;            // limbs to write
     unsigned int *ticket;       // dynamic tile counter (zeroed per launch)
     unsigned int *status;       // per-tile look-back words (zeroed per launch)

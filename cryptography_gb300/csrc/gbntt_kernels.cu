@@ -224,13 +224,13 @@ __device__ __forceinline__ void garner2_vals(const CarryArgs &a, uint64_t r0, ui
     if ((long long)top >= a.n_coef) err |= ERR_GARNER_DIGIT;
 }
 
-// The 31-bit prime set. A true coefficient is below n_coef 2^64: a larger top
+// The 31-bit prime set. A true coefficient is below limit 2^64: a larger top
 // word means corrupted residues.
 __device__ __forceinline__ void garner31_vals(const CarryArgs &a, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t &w0,
                                               uint32_t &w1, uint32_t &w2, unsigned &err)
 {
     garner31(r0, r1, r2, w0, w1, w2);
-    if ((long long)w2 >= a.n_coef) err |= ERR_GARNER_DIGIT;
+    if ((long long)w2 >= a.limit) err |= ERR_GARNER_DIGIT;
 }
 
 template <int SET>
@@ -290,6 +290,7 @@ __global__ void __launch_bounds__(kCarryThreads, GBNTT_CARRY_MIN_BLOCKS) garner_
         a.out = a.out_tab[b];
         a.n_out = a.nout_tab[b];
         a.n_coef = n_prod;
+        a.limit = n_prod;
         a.status += a.tile_start[b];
     }
     const long long tile = BATCH ? (long long)s_tile - a.tile_start[s_prod] : (long long)s_tile;

@@ -16,7 +16,9 @@
 // All three primes have 2-adicity of at least 25 and p - 1 divisible by 3:
 //   15 2^27 + 1, 27 2^26 + 1, 63 2^25 + 1,
 // so transforms have up to 2^25 points, or 3 2^k with k <= 25. Longer
-// products use the 64-bit prime sets.
+// products (up to 2^29 coefficients) are put together from up to 16
+// transforms of 2^25 points (gbntt_p31_outer.cu); beyond that the modulus is
+// too small and the 64-bit prime sets take over.
 //
 // One launch covers all three primes (the prime is the fastest block index,
 // so the CTAs that read the same limbs or tile run side by side), and both
@@ -315,6 +317,20 @@ struct P31R3Args {
     ShoupWord c[3], step[3];            // (om - om^2) / 2; w^G (forward) or w^-G (inverse), G = blocks x 256
 };
 cudaError_t launch_p31_radix3(bool inverse, const P31R3Args &a, cudaStream_t st);
+
+// Outer stage of a product of up to R 2^25 coefficients: spectrum m at
+// spec[prime] + m 2^25.
+constexpr int kP31MaxOuter = 16;
+struct P31OuterArgs {
+    uint32_t *spec[3];
+    const uint32_t *limbs;              // forward input
+    long long n_limbs;
+    int blocks;                         // ceil(n_limbs / 2^25), at most R
+    const uint32_t *g[3];               // two-level tables of g (forward) or g^-1: 2^10 words g^(i 2^15), 2^15 words g^i
+};
+cudaError_t launch_p31_outer(int R, bool inverse, const P31OuterArgs &a, cudaStream_t st);
+uint64_t p31_outer_root(int k);         // g of prime k
+cudaError_t p31_outer_init();
 
 // A whole product of up to 2^kP31BlockLog coefficients in one CTA (W of them:
 // the tables, one CTA each).

@@ -211,7 +211,7 @@ def plan(log_n):
 
 
 LAUNCH_KINDS = ("fwd_pass_first", "fwd_pass", "inv_pass_first", "inv_pass", "garner_carry", "fused_inner_pass",
-                "radix3_fwd", "radix3_inv", "block_product")
+                "radix3_fwd", "radix3_inv", "block_product", "outer_fwd", "outer_inv")
 
 
 def launch_log(enable):
