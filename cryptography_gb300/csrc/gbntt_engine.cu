@@ -97,7 +97,7 @@ struct Engine {
     uint32_t *d_tw31 = nullptr;     // its two-level tables: [prime][dir][2^10 hi | 2^15 lo], Montgomery form
     uint32_t *d_rho31 = nullptr;    // radix-3: [prime][3 2^10 hi | 2^15 lo]
     uint32_t *d_blk31 = nullptr;    // block kernel: [prime][dir], 2^(L + 1) words per length from offset 2^(L + 1)
-    uint32_t *d_g31 = nullptr;      // outer stage: [prime][dir][2^10 hi | 2^15 lo] powers of g, Montgomery form
+    uint32_t *d_g31 = nullptr;      // outer stage: [g, g^(d/2)][prime][dir][2^10 hi | 2^15 lo], Montgomery form
     ShoupWord r3c31[3] = {};        // (om - om^2) / 2 per prime
     uint64_t rho31[3] = {};         // rho (order 3 2^25) per prime
     bool batch_split = true;        // uneven batch products split into chunk products
@@ -370,7 +370,7 @@ static size_t workspace_bytes(int max_log)
     const size_t tw = 4 * 2 * 2 * (size_t)kTwSize * sizeof(uint64_t) + 2 * 2 * (size_t)kTwSize * sizeof(uint32_t) +
                       4 * 2 * (size_t)kStep1Words * sizeof(uint64_t) + 2 * (size_t)kStep1Words * sizeof(uint32_t) +
                       4 * (size_t)kTwSize * (2 * sizeof(uint64_t) + sizeof(uint32_t)) +   // radix-3 rho tables
-                      6 * (size_t)kP31StepWords * sizeof(ShoupWord) + (12 * kTw31Words + 3 * kRho31Words + 6 * kBlk31Words) * sizeof(uint32_t);
+                      6 * (size_t)kP31StepWords * sizeof(ShoupWord) + (18 * kTw31Words + 3 * kRho31Words + 6 * kBlk31Words) * sizeof(uint32_t);
     const size_t ctl = (2 + status_words(n)) * sizeof(unsigned);
     const size_t io = (4 * n + 64) * sizeof(uint32_t);
     return spec + tw + ctl + io;
@@ -417,7 +417,7 @@ static cudaError_t init_p31()
 {
     constexpr int kHi = 1 << (kP31MaxLog - kTwBits);
     std::vector<ShoupWord> st(6 * (size_t)kP31StepWords, ShoupWord{0, 0});
-    std::vector<uint32_t> tw(6 * kTw31Words), rt(3 * kRho31Words), blk(6 * kBlk31Words), gt(6 * kTw31Words);
+    std::vector<uint32_t> tw(6 * kTw31Words), rt(3 * kRho31Words), blk(6 * kBlk31Words), gt(12 * kTw31Words);
     for (int k = 0; k < 3; k++) {
         const uint64_t p = kP31[k];
         auto mont = [&](uint64_t x) { return (uint32_t)((x << 32) % p); };
@@ -429,13 +429,15 @@ static cudaError_t init_p31()
             for (int i = 0; i < kHi; i++) { t[i] = mont(x); x = x * big % p; }
             x = 1;
             for (int i = 0; i < kTwSize; i++) { t[kHi + i] = mont(x); x = x * wd % p; }
-            const uint64_t gd = dir ? p31_pow(p31_outer_root(k), p - 2, p) : p31_outer_root(k);
-            const uint64_t gbig = p31_pow(gd, kTwSize, p);
-            t = gt.data() + ((size_t)k * 2 + dir) * kTw31Words;
-            x = 1;
-            for (int i = 0; i < kHi; i++) { t[i] = mont(x); x = x * gbig % p; }
-            x = 1;
-            for (int i = 0; i < kTwSize; i++) { t[kHi + i] = mont(x); x = x * gd % p; }
+            for (int half = 0; half < 2; half++) {
+                const uint64_t root = half ? p31_outer_half(k) : p31_outer_root(k);
+                const uint64_t gd = dir ? p31_pow(root, p - 2, p) : root, gbig = p31_pow(gd, kTwSize, p);
+                t = gt.data() + (((size_t)half * 3 + k) * 2 + dir) * kTw31Words;
+                x = 1;
+                for (int i = 0; i < kHi; i++) { t[i] = mont(x); x = x * gbig % p; }
+                x = 1;
+                for (int i = 0; i < kTwSize; i++) { t[kHi + i] = mont(x); x = x * gd % p; }
+            }
             for (int l = kMinLog; l <= kP31BlockLog; l++)
                 p31_block_tables(l, blk.data() + ((size_t)k * 2 + dir) * kBlk31Words + ((size_t)2 << l),
                                  p31_pow(wd, 1ull << (kP31MaxLog - l), p), p);
@@ -1126,6 +1128,7 @@ static int p31_outer(const P31Op &op, size_t stride, int R, bool inverse, cudaSt
     for (int k = 0; k < 3; k++) {
         a.spec[k] = (uint32_t *)(op.spec + k * stride);
         a.g[k] = g.d_g31 + ((size_t)k * 2 + (inverse ? 1 : 0)) * kTw31Words;
+        a.gh[k] = a.g[k] + 6 * kTw31Words;
     }
     const double nbw = 12.0 * (double)R * (double)((size_t)1 << kP31MaxLog);
     rec_begin(st, inverse ? 10 : 9, R, inverse ? 2.0 * nbw : nbw + 4.0 * (double)op.n);

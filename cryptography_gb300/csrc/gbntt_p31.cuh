@@ -327,9 +327,11 @@ struct P31OuterArgs {
     long long n_limbs;
     int blocks;                         // ceil(n_limbs / 2^25), at most R
     const uint32_t *g[3];               // two-level tables of g (forward) or g^-1: 2^10 words g^(i 2^15), 2^15 words g^i
+    const uint32_t *gh[3];              // the same of g^(d / 2) (primes whose d is even)
 };
 cudaError_t launch_p31_outer(int R, bool inverse, const P31OuterArgs &a, cudaStream_t st);
 uint64_t p31_outer_root(int k);         // g of prime k
+uint64_t p31_outer_half(int k);         // g^(d / 2)
 cudaError_t p31_outer_init();
 
 // A whole product of up to 2^kP31BlockLog coefficients in one CTA (W of them:

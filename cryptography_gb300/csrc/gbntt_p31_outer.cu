@@ -10,6 +10,10 @@
 //            under X -> g^m X, a cyclic convolution of length M)
 //   inverse  t_m = z_m[j] g^(-jm), x[j + r M] = sum_m V^-1[r][m] t_m with the
 //            Vandermonde matrix V[m][r] = gamma^(rm).
+// Two of the primes have -1 among the M-th powers (d even): there, for even
+// R, the c_m are pairs +-gamma^i, and the even- and odd-indexed blocks are
+// two sums of half the length, added and subtracted (forward 80 to 60, inverse
+// 112 to 80 cycles per residue, warp and SM sub-partition at R = 16).
 // A dense R x R product instead of log2 R radix-2 levels: one wide multiply
 // per term, the high word folded every second term, one Montgomery reduction
 // per sum. It costs about as much as 8 levels of the pass chain at R = 16 (of
@@ -51,7 +55,10 @@ constexpr ForwardMatrix forward_matrix()
     return f;
 }
 __constant__ const ForwardMatrix c_fwd = forward_matrix();
-// V^-1 for each R, Montgomery form, row r at [R][k][r kMaxR + m]
+// V^-1 for each R, Montgomery form, row r at [R][k][r kMaxR + m]; for paired
+// points the two matrices of R / 2 rows that take the pairs' sums to the
+// even blocks ([s kMaxR + i]) and their differences to the odd ones
+// ([s kMaxR + kMaxR / 2 + i])
 __constant__ uint32_t c_inv[kMaxR + 1][3][kMaxR * kMaxR];
 
 struct Acc {
@@ -70,6 +77,8 @@ struct Acc {
         return __viaddmin_u32(d, p, d);
     }
 };
+
+__host__ __device__ constexpr bool outer_paired(int R, int k) { return R % 2 == 0 && k < 2; }
 
 // g^(+-j), Montgomery form
 __device__ __forceinline__ uint32_t g_pow(const uint32_t *t, uint32_t j, uint32_t p, uint32_t pinv)
@@ -97,6 +106,35 @@ __global__ void __launch_bounds__(256) p31_outer_fwd_kernel(const __grid_constan
     const uint32_t w1 = g_pow(a.g[k], j, p, pinv);
     uint32_t w = w1;
     uint32_t *out = a.spec[k] + j;
+    if (outer_paired(R, k)) {
+        const uint32_t h = g_pow(a.gh[k], j, p, pinv);   // g^(j d / 2): the twist between a pair's points
+#pragma unroll
+        for (int i = 0; i < R / 2; i++) {
+            Acc even, odd;
+#pragma unroll
+            for (int r0 = 0; r0 < R; r0 += 4)
+                if (r0 == 0 || r0 < ni) {
+#pragma unroll
+                    for (int r = r0; r < r0 + 4 && r < R; r += 2) {
+                        even.add(x[r], c_fwd.v[k][i][r]);
+                        odd.add(x[r + 1], c_fwd.v[k][i][r + 1]);
+                    }
+                    even.fold(p);
+                    odd.fold(p);
+                }
+            const uint32_t e = even.reduce(p, pinv), o = odd.reduce(p, pinv);
+            const uint32_t y0 = p31_add(e, o, p), y1 = p31_sub(e, o, p);
+            if (i == 0) {
+                out[0] = y0;
+                out[kM] = p31_mont(y1, h, p, pinv);
+            } else {
+                out[(size_t)(2 * i) * kM] = p31_mont(y0, w, p, pinv);
+                out[(size_t)(2 * i + 1) * kM] = p31_mont(y1, p31_mont(w, h, p, pinv), p, pinv);
+                if (i < R / 2 - 1) w = p31_mont(w, w1, p, pinv);
+            }
+        }
+        return;
+    }
 #pragma unroll
     for (int m = 0; m < R; m++) {
         Acc s;
@@ -131,6 +169,28 @@ __global__ void __launch_bounds__(256) p31_outer_inv_kernel(const __grid_constan
 #pragma unroll
     for (int m = 0; m < R; m++) t[m] = z[(size_t)m * kM];
     uint32_t w = w1;
+    if (outer_paired(R, k)) {
+        const uint32_t h = g_pow(a.gh[k], j, p, pinv);
+#pragma unroll
+        for (int i = 0; i < R / 2; i++) {
+            const uint32_t y0 = i ? p31_mont(t[2 * i], w, p, pinv) : t[0];
+            const uint32_t y1 = p31_mont(t[2 * i + 1], i ? p31_mont(w, h, p, pinv) : h, p, pinv);
+            if (i > 0 && i < R / 2 - 1) w = p31_mont(w, w1, p, pinv);
+            t[2 * i] = p31_add(y0, y1, p);
+            t[2 * i + 1] = p31_sub(y0, y1, p);
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            Acc s;
+#pragma unroll
+            for (int i = 0; i < R / 2; i++) {
+                s.add(t[2 * i + (r & 1)], c_inv[R][k][(r / 2) * kMaxR + (r & 1) * (kMaxR / 2) + i]);
+                if ((i & 1) || i == R / 2 - 1) s.fold(p);
+            }
+            z[(size_t)r * kM] = s.reduce(p, pinv);
+        }
+        return;
+    }
 #pragma unroll
     for (int m = 1; m < R; m++) {
         t[m] = p31_mont(t[m], w, p, pinv);
@@ -179,30 +239,49 @@ cudaError_t launch_p31_outer(int R, bool inverse, const P31OuterArgs &a, cudaStr
 }
 
 uint64_t p31_outer_root(int k) { return outer_g(k); }
+uint64_t p31_outer_half(int k) { return k < 2 ? p31_pow(outer_g(k), outer_order(k) / 2, kP31[k]) : 1; }
 
-// The inverse Vandermonde matrices: row r, column m of V^-1 is the X^r
-// coefficient of the Lagrange polynomial prod_(i != m) (X - c_i) / (c_m - c_i).
+// V^-1 for the n points c mod p: row r, column m is the X^r coefficient of
+// the Lagrange polynomial prod_(i != m) (X - c_i) / (c_m - c_i).
+static std::vector<uint64_t> vandermonde_inverse(const std::vector<uint64_t> &c, uint64_t p)
+{
+    const int n = (int)c.size();
+    std::vector<uint64_t> all(n + 1, 0), v((size_t)n * n);
+    all[0] = 1;   // prod (X - c_i), all[d] the X^d coefficient
+    for (int m = 0; m < n; m++)
+        for (int d = m + 1; d >= 0; d--) all[d] = ((d ? all[d - 1] : 0) + all[d] * (p - c[m])) % p;
+    for (int m = 0; m < n; m++) {
+        std::vector<uint64_t> q(n);   // divided by X - c_m
+        uint64_t carry = 0, denom = 1;
+        for (int d = n; d >= 1; d--) q[d - 1] = carry = (all[d] + carry * c[m]) % p;
+        for (int i = 0; i < n; i++)
+            if (i != m) denom = denom * ((c[m] + p - c[i]) % p) % p;
+        const uint64_t inv = p31_pow(denom, p - 2, p);
+        for (int r = 0; r < n; r++) v[(size_t)r * n + m] = q[r] * inv % p;
+    }
+    return v;
+}
+
 cudaError_t p31_outer_init()
 {
     std::vector<uint32_t> h((size_t)(kMaxR + 1) * 3 * kMaxR * kMaxR, 0);
     for (int R = 2; R <= kMaxR; R++)
         for (int k = 0; k < 3; k++) {
             const uint64_t p = kP31[k], gamma = p31_pow(outer_g(k), kM, p);
-            std::vector<uint64_t> c(R), all(R + 1, 0);
-            for (int m = 0; m < R; m++) c[m] = p31_pow(gamma, (uint64_t)m, p);
-            all[0] = 1;   // prod (X - c_i), all[d] the X^d coefficient
-            for (int m = 0; m < R; m++)
-                for (int d = m + 1; d >= 0; d--) all[d] = ((d ? all[d - 1] : 0) + all[d] * (p - c[m])) % p;
-            for (int m = 0; m < R; m++) {
-                std::vector<uint64_t> q(R);   // divided by X - c_m
-                uint64_t carry = 0, denom = 1;
-                for (int d = R; d >= 1; d--) q[d - 1] = carry = (all[d] + carry * c[m]) % p;
-                for (int i = 0; i < R; i++)
-                    if (i != m) denom = denom * ((c[m] + p - c[i]) % p) % p;
-                const uint64_t inv = p31_pow(denom, p - 2, p);
-                for (int r = 0; r < R; r++)
-                    h[(((size_t)R * 3 + k) * kMaxR + r) * kMaxR + m] = (uint32_t)(((q[r] * inv % p) << 32) % p);
-            }
+            uint32_t *dst = h.data() + ((size_t)R * 3 + k) * kMaxR * kMaxR;
+            auto mont = [&](uint64_t x) { return (uint32_t)((x << 32) % p); };
+            const bool paired = outer_paired(R, k);
+            const int n = paired ? R / 2 : R;
+            std::vector<uint64_t> c(n);
+            for (int m = 0; m < n; m++) c[m] = p31_pow(gamma, (uint64_t)m * (paired ? 2 : 1), p);
+            const std::vector<uint64_t> v = vandermonde_inverse(c, p);
+            for (int r = 0; r < n; r++)
+                for (int m = 0; m < n; m++) {
+                    const uint64_t x = v[(size_t)r * n + m], half = x * ((p + 1) / 2) % p;
+                    dst[r * kMaxR + m] = mont(paired ? half : x);
+                    if (paired)   // the differences are 2 gamma^m times the odd blocks' polynomial
+                        dst[r * kMaxR + kMaxR / 2 + m] = mont(half * p31_pow(p31_pow(gamma, (uint64_t)m, p), p - 2, p) % p);
+                }
         }
     return cudaMemcpyToSymbol(c_inv, h.data(), h.size() * sizeof(uint32_t));
 }
