@@ -450,6 +450,9 @@ static cudaError_t init_p31()
                         s[L - 32 + ka * B + b] = s[kStep1Words + L - 32 + b * A + ka] =
                             shoup_word(p31_pow(wl, (uint64_t)ka * b, p), p);
             }
+            const uint64_t w512 = p31_pow(wd, 1ull << (kP31MaxLog - 9), p), w64 = p31_pow(w512, 8, p);
+            for (int i = 0; i < 512; i++) s[kP31Step9 + i] = shoup_word(p31_pow(w512, (uint64_t)(i >> 6) * (i & 63), p), p);
+            for (int i = 0; i < 64; i++) s[kP31Step9 + 512 + i] = shoup_word(p31_pow(w64, (uint64_t)(i >> 3) * (i & 7), p), p);
         }
         const uint64_t rho = p31_pow(kP31Gen[k], (p - 1) / (3ull << kP31MaxLog), p), big = p31_pow(rho, kTwSize, p);
         uint32_t *t = rt.data() + k * kRho31Words;

@@ -162,13 +162,21 @@ constexpr int p31_bitrev(int x, int bits)
 }
 
 // Radix-2 DIF DFT of 2^LOG_R points in registers: X[k] ends in
-// x[bitrev(k)]. roots: w_32^i of the prime and direction.
+// x[bitrev(k)]. roots: w_32^i of the prime and direction. upper_zero: the
+// upper half of x is zero and not read (a first pass over an operand of at
+// most half the transform's length).
 template <int LOG_R>
-__device__ __forceinline__ void p31_dft(uint32_t *x, const ShoupWord *roots, uint32_t p)
+__device__ __forceinline__ void p31_dft(uint32_t *x, const ShoupWord *roots, uint32_t p, bool upper_zero = false)
 {
     constexpr int R = 1 << LOG_R;
+    if (upper_zero) {
+        x[R / 2] = x[0];
+#pragma unroll
+        for (int i = 1; i < R / 2; i++) x[R / 2 + i] = p31_shoup(x[i], roots[i * (32 / R)], p);
+    }
 #pragma unroll
     for (int s = R / 2; s >= 1; s >>= 1) {
+        if (s == R / 2 && upper_zero) continue;
 #pragma unroll
         for (int blk = 0; blk < R; blk += 2 * s) {
 #pragma unroll
@@ -269,8 +277,11 @@ __device__ __forceinline__ void p31_tile_inv(uint32_t *x, uint32_t *sm, int g, i
 
 // Step tables of one prime and direction: for pass size 2^l the A x B block
 // at 2^l - 32 holds w_L^(ka b) at [ka B + b]; the second half (at
-// kStep1Words) the same at [b A + ka].
-constexpr int kP31StepWords = 2 * kStep1Words;
+// kStep1Words) the same at [b A + ka]. After them the tables of the strided
+// 2^9-point passes' three steps: w_512^(k0 c) at [64 k0 + c], then
+// w_64^(k1 m0) at [8 k1 + m0].
+constexpr int kP31Step9 = 2 * kStep1Words;
+constexpr int kP31StepWords = kP31Step9 + 512 + 64;
 
 struct P31PassArgs {
     uint32_t *data[2][3];               // per operand (blockIdx.y) and prime

@@ -20,6 +20,10 @@ namespace {
 // 2^17 points the halved number of tiles costs more, 27.0 and 35.1 us.
 constexpr long long kTwoColumns = 1LL << 20;
 
+// ... and four of them in 2^9-point passes (2^17 points 18.5 us per product
+// with one, 22.4 with four).
+constexpr long long kFourColumns = 1LL << 21;
+
 // word at byte offset off of a base address
 template <class Word>
 __device__ __forceinline__ Word ld_off(const void *base, uint32_t off)
@@ -234,6 +238,177 @@ p31_pass_kernel(const __grid_constant__ P31PassArgs a)
     }
 }
 
+// Passes of 2^9 points: three steps of 8-point DFTs over four adjacent
+// columns per thread, 32 columns per CTA (rows of 128 bytes). As 32 x 16
+// points a thread holds 32 residues of one column, pays for its own addresses
+// and loads (62 instructions per residue of a first pass, 54 of an inverse
+// one; here 53 and 43) and reads rows of 64 bytes. An operand of at most half
+// the transform's length leaves the upper half of step 1 zero. Measured at
+// 2^25 points: first pass of both operands 444 -> 416 us, inverse 222 -> 207
+// us; two columns of 64-byte rows with the same steps were slower (565 and
+// 248 us), and so was skipping the zero half in 2^8-point passes.
+// Row m = 64 m2 + 8 m1 + m0; step 1 transforms over m2 (k0 comes out), step 2
+// over m1 (k1), step 3 over m0 (k2); the output row is k0 + 8 k1 + 64 k2.
+// Exchange word (16 bytes) (k0, m1 | k1, m0) at ((8 k0 + m1) 8 + m0) GP + gp:
+// the 8 threads that one access serves are adjacent.
+__device__ __forceinline__ uint32_t word4(const uint4 &w, int v)
+{
+    return v == 0 ? w.x : v == 1 ? w.y : v == 2 ? w.z : w.w;
+}
+
+template <int DIR, bool LIMBS>
+__global__ void __launch_bounds__(512, 2) p31_pass9_kernel(const __grid_constant__ P31PassArgs a)
+{
+    constexpr int GP = 8, V = 4;
+    extern __shared__ uint4 sm9[];
+    const int k = blockIdx.x % 3, op = blockIdx.y;
+    const long long col0 = (long long)(blockIdx.x / 3) * (V * GP);
+    const uint32_t p = p31_prime(k), pinv = p31_inv(k);
+    const int t = threadIdx.x, gp = t & (GP - 1), q = t >> 3;
+    const int log_s = a.log_s;
+    const uint32_t sub0 = (uint32_t)((col0 >> log_s) << a.log_m);
+    const uint32_t j = (uint32_t)(col0 & ((1LL << log_s) - 1)) + V * gp;
+    uint32_t *data = a.data[op][k];
+    const uint32_t step = 256u << log_s;   // 64 rows, in bytes
+    const uint32_t off0 = (sub0 + j + ((uint32_t)q << log_s)) << 2;
+    uint32_t x[V][8];
+    bool upper_zero = false;
+    chain_wait();
+    if (LIMBS) {
+        const uint32_t *limbs;
+        long long n;
+        if (a.limb_tab[op]) {
+            const long long b = (long long)(sub0 >> a.log_prod);
+            limbs = a.limb_tab[op][b];
+            n = a.len_tab[op][b];
+        } else {
+            limbs = a.limbs[op];
+            n = a.n_limbs[op];
+        }
+        const uint32_t nn = (uint32_t)n, r0 = j + ((uint32_t)q << log_s);
+        upper_zero = 2 * n <= 1LL << a.log_m;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (h == 1 && upper_zero) break;
+#pragma unroll
+            for (int i = 4 * h; i < 4 * h + 4; i++)
+#pragma unroll
+                for (int v = 0; v < V; v++) {
+                    const uint32_t r = r0 + ((uint32_t)(64 * i) << log_s) + v;
+                    x[v][i] = r < nn ? __ldg(limbs + r) : 0u;
+                }
+#pragma unroll
+            for (int i = 4 * h; i < 4 * h + 4; i++)
+#pragma unroll
+                for (int v = 0; v < V; v++) x[v][i] = p31_limb(x[v][i], p);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint4 w = ld_off<uint4>(data, off0 + i * step);
+#pragma unroll
+            for (int v = 0; v < V; v++) x[v][i] = word4(w, v);
+        }
+    }
+    const uint32_t *ptw = a.ptw[k];
+    const void *tb = reinterpret_cast<const void *>(reinterpret_cast<uintptr_t>(ptw) - ((uintptr_t)sub0 << 2));
+    const int sh = kP31MaxLog - a.log_m;
+    // pass twiddles of rows r0 + 64 i at byte offset off + i step
+    auto twiddle = [&](uint32_t off, int r0) {
+        if (ptw) {
+#pragma unroll
+            for (int i0 = 0; i0 < 8; i0 += 4) {
+                uint4 tw[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) tw[i] = ldg_off<uint4>(tb, off + (i0 + i) * step);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int v = 0; v < V; v++) x[v][i0 + i] = p31_mont(x[v][i0 + i], word4(tw[i], v), p, pinv);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int v = 0; v < V; v++) {
+                    uint32_t w = p31_tw(a, k, (uint32_t)(((uint64_t)(r0 + 64 * i) * (j + v)) << sh), p, pinv);
+                    if (DIR == 1 && a.use_scale) w = p31_mont(w, a.scale[k], p, pinv);
+                    x[v][i] = p31_mont(x[v][i], w, p, pinv);
+                }
+        }
+    };
+    if (DIR == 1) twiddle(off0, q);
+    const ShoupWord *roots = c_p31_roots.v[k][DIR];
+    const ShoupWord *__restrict__ st = a.st[k] + kP31Step9;   // w_512^(k0 c) at [64 k0 + c], then w_64^(k1 m0) at [8 k1 + m0]
+    // one step's DFTs with its twiddles f[k by], results to w[k stride]
+    auto dfts = [&](bool zero) {
+#pragma unroll
+        for (int v = 0; v < V; v++) p31_dft<3>(x[v], roots, p, zero);
+    };
+    auto put = [&](uint4 *w, int stride, const ShoupWord *f, int by) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int at = p31_bitrev(i, 3);
+            uint4 y = make_uint4(x[0][at], x[1][at], x[2][at], x[3][at]);
+            if (i > 0) {
+                const ShoupWord s = f[i * by];
+                y = make_uint4(p31_shoup(y.x, s, p), p31_shoup(y.y, s, p), p31_shoup(y.z, s, p), p31_shoup(y.w, s, p));
+            }
+            w[i * stride] = y;
+        }
+    };
+    auto get = [&](const uint4 *w, int stride) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint4 y = w[i * stride];
+#pragma unroll
+            for (int v = 0; v < V; v++) x[v][i] = word4(y, v);
+        }
+    };
+    dfts(LIMBS && upper_zero);
+    put(sm9 + q * GP + gp, 64 * GP, st + q, 64);
+    __syncthreads();
+    uint4 *const w2 = sm9 + ((q >> 3) * 64 + (q & 7)) * GP + gp;   // (k0, m0)
+    get(w2, 8 * GP);
+    dfts(false);
+    put(w2, 8 * GP, st + 512 + (q & 7), 8);
+    __syncthreads();
+    get(sm9 + q * 8 * GP + gp, GP);   // (k0, k1) = (q >> 3, q & 7)
+    const int row = (q >> 3) + 8 * (q & 7);
+    const uint32_t out0 = (sub0 + j + ((uint32_t)row << log_s)) << 2;
+    dfts(false);
+    {
+        uint32_t y[V][8];
+#pragma unroll
+        for (int v = 0; v < V; v++)
+#pragma unroll
+            for (int i = 0; i < 8; i++) y[v][i] = x[v][p31_bitrev(i, 3)];
+#pragma unroll
+        for (int v = 0; v < V; v++)
+#pragma unroll
+            for (int i = 0; i < 8; i++) x[v][i] = y[v][i];
+    }
+    if (DIR == 0) twiddle(out0, row);
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        st_off<uint4>(data, out0 + i * step, make_uint4(x[0][i], x[1][i], x[2][i], x[3][i]));
+}
+
+cudaError_t launch_9(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
+{
+    constexpr size_t smem = 64 * 64 * sizeof(uint4);
+    static const cudaError_t attr[3] = {
+        cudaFuncSetAttribute(p31_pass9_kernel<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+        cudaFuncSetAttribute(p31_pass9_kernel<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+        cudaFuncSetAttribute(p31_pass9_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)};
+    for (const cudaError_t e : attr)
+        if (e != cudaSuccess) return e;
+    return launch_chained(dir == 1 ? p31_pass9_kernel<1, false>
+                          : limbs  ? p31_pass9_kernel<0, true>
+                                   : p31_pass9_kernel<0, false>,
+                          dim3((unsigned)(3 * (a.ncols / 32)), (unsigned)nops), 512, smem, st, a);
+}
+
 template <int LOG_L, int V>
 cudaError_t launch_v(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
 {
@@ -278,7 +453,7 @@ cudaError_t launch_p31_pass(int log_l, int dir, bool limbs, int nops, const P31P
     case 6: return launch_l<6>(dir, limbs, nops, a, st);
     case 7: return launch_l<7>(dir, limbs, nops, a, st);
     case 8: return launch_l<8>(dir, limbs, nops, a, st);
-    case 9: return launch_l<9>(dir, limbs, nops, a, st);
+    case 9: return (a.ncols << 9) * nops >= kFourColumns ? launch_9(dir, limbs, nops, a, st) : launch_l<9>(dir, limbs, nops, a, st);
     case 10: return launch_l<10>(dir, limbs, nops, a, st);
     default: return cudaErrorInvalidValue;
     }
