@@ -754,6 +754,15 @@ static int p31_outer_blocks(size_t na, size_t nb)
     return g.p31 && g.prime_set == 2 && fits ? (int)blocks : 0;
 }
 
+// Whether a product of 32-bit limbs that fits the engine runs on the 31-bit
+// primes (in mul_dev).
+static int r3_log(size_t na, size_t nb);
+static bool on_p31(size_t na, size_t nb)
+{
+    const int k3 = r3_log(na, nb);
+    return use_p31(k3 >= g.r3_min_log ? k3 : choose_log(na, nb)) || p31_outer_blocks(na, nb) > 0;
+}
+
 // Whether a product of transform length 2^L runs in one CTA.
 static bool use_block(int L) { return use_p31(L) && L <= kP31BlockLog; }
 
@@ -1514,6 +1523,11 @@ static int mul_dev64(uint64_t *d_c, const uint64_t *d_a, size_t na, const uint64
         set_err("product needs %zu coefficients but the engine was initialised for 2^%d", na + nb - 1, g.max_log);
         return GBNTT_ERR_SIZE;
     }
+    // The same integers as 32-bit limbs, where the 31-bit primes take them:
+    // twice the coefficients, but three 31-bit residues each instead of three
+    // 64-bit ones (700001 x 600011 limbs 500 -> 181 us).
+    if (2 * (na + nb) - 1 <= g.n_max && on_p31(2 * na, 2 * nb))
+        return mul_dev((uint32_t *)d_c, (const uint32_t *)d_a, 2 * na, (const uint32_t *)d_b, 2 * nb, st);
     const bool square = (d_a == d_b && na == nb);
     uint64_t *specA = g.d_spec;
     uint64_t *specB = g.d_spec + 3 * g.n_max;
