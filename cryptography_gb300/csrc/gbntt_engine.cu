@@ -92,6 +92,7 @@ struct Engine {
     uint64_t r3c[5] = {};           // per prime: c = (om - om^2) / 2 in its multiply form
     uint64_t r3rho[5] = {};         // per prime: rho (order 3 2^30), plain
     int r3_min_log = 20;            // radix-3 for c products of 3 2^k points when c 2^k >= 2^r3_min_log
+    int r3_alone_log = 17;          // ... and on the 31-bit primes from 2^k = 2^r3_alone_log for any of them
     bool p31 = true;                // 31-bit prime set where it fits
     ShoupWord *d_st31 = nullptr;    // its step tables: [prime][dir][kP31StepWords]
     uint32_t *d_tw31 = nullptr;     // its two-level tables: [prime][dir][2^10 hi | 2^15 lo], Montgomery form
@@ -702,6 +703,7 @@ static int init_impl(int max_log)
         g.radix3 = !(r3 && r3[0] == '0');
         const char *r3m = getenv("GBNTT_RADIX3_MIN_LOG");
         g.r3_min_log = r3m ? std::max(10, std::min(30, atoi(r3m))) : 20;
+        g.r3_alone_log = r3m ? g.r3_min_log : 17;
         const char *pt = getenv("GBNTT_PASS_TABLES");
         g.pass_tables = !(pt && pt[0] == '0');
         const char *pb = getenv("GBNTT_PASS_TABLES_MB");
@@ -754,13 +756,19 @@ static int p31_outer_blocks(size_t na, size_t nb)
     return g.p31 && g.prime_set == 2 && fits ? (int)blocks : 0;
 }
 
+// Whether a product alone takes 3 2^k points instead of 2^(k+2). On the
+// 31-bit primes, measured: 3 2^16 points 25.0 us against 25.2, 3 2^17 32.1
+// against 35.4, 3 2^18 50 against 57, 3 2^20 172 against 193, 3 2^14 19.8
+// against 15.3; on q0 with p3 see r3_log.
+static bool r3_alone(int k) { return k >= (use_p31(k) ? g.r3_alone_log : g.r3_min_log); }
+
 // Whether a product of 32-bit limbs that fits the engine runs on the 31-bit
 // primes (in mul_dev).
 static int r3_log(size_t na, size_t nb);
 static bool on_p31(size_t na, size_t nb)
 {
     const int k3 = r3_log(na, nb);
-    return use_p31(k3 >= g.r3_min_log ? k3 : choose_log(na, nb)) || p31_outer_blocks(na, nb) > 0;
+    return use_p31(r3_alone(k3) ? k3 : choose_log(na, nb)) || p31_outer_blocks(na, nb) > 0;
 }
 
 // Whether a product of transform length 2^L runs in one CTA.
@@ -1107,15 +1115,12 @@ static int p31_radix3(const P31Op &op, size_t stride, int k3, bool inverse, cuda
     a.M = 1LL << k3;
     a.W = op.W;
     a.shift = kP31MaxLog - k3;
-    const long long per_block = 256LL * kR3Unroll;
-    a.blocks = (int)((a.M + per_block - 1) / per_block);
     a.limbs = op.limbs;
     a.n_limbs = (long long)op.n;
     a.limb_tab = op.limb_tab;
     a.len_tab = op.len_tab;
     const uint64_t order = 3ull << kP31MaxLog;
-    uint64_t e = ((256ull * a.blocks) << a.shift) % order;
-    if (inverse && e) e = order - e;
+    const uint64_t e = inverse ? order - (1ull << a.shift) : 1ull << a.shift;
     for (int k = 0; k < 3; k++) {
         a.spec[k] = (uint32_t *)(op.spec + k * stride);
         a.rho[k] = g.d_rho31 + k * kRho31Words;
@@ -1258,7 +1263,8 @@ struct StageJob {
 // (measured per product against the next power of two: 3 2^18 points
 // 1.02 x, 3 2^19 0.99 x, 3 2^20 0.84 x, 3 2^22 0.81 x, 3 2^24 0.79 x): a
 // product alone takes it from k = r3_min_log, a batch for c products of one
-// length when c 2^k >= 2^r3_min_log (batch_mul).
+// length when c 2^k >= 2^r3_min_log (batch_mul). (These are q0 with p3; the
+// 31-bit primes' products alone: r3_alone.)
 static int r3_log(size_t na, size_t nb)
 {
     if (!g.radix3 || g.prime_set != 2 || na == 0 || nb == 0) return -1;
@@ -1446,7 +1452,7 @@ static int mul_dev(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint32_t
         return GBNTT_ERR_SIZE;
     }
     const int k3 = r3_log(na, nb);
-    const bool r3 = k3 >= g.r3_min_log;
+    const bool r3 = r3_alone(k3);
     if (use_p31(r3 ? k3 : L)) return mul_dev_p31(d_c, d_a, na, d_b, nb, r3 ? k3 : L, r3 ? 3 : 1, st, stage_b, stage_a);
     if (const int R = p31_outer_blocks(na, nb))
         return mul_dev_p31(d_c, d_a, na, d_b, nb, kP31MaxLog, R, st, stage_b, stage_a);
@@ -1937,7 +1943,7 @@ static int batch_mul(uint32_t *const *d_c, const uint32_t *const *d_a, const siz
         // products (not cyclic, not a split's chunk) take a transform of
         // 3 2^k points where it is shorter than the power of two and there
         // is enough of them: c products of 3 2^k points with
-        // c 2^k >= 2^r3_min_log. A pair takes it for both or neither (its
+        // c 2^k >= 2^r3_min_log, or any that would take it alone. A pair takes it for both or neither (its
         // right operand's transform is shared); a run sharing one right
         // operand is split by length as before, each length's wave sharing it.
         std::vector<int> k3s(all.size(), -1);
@@ -1961,7 +1967,7 @@ static int batch_mul(uint32_t *const *d_c, const uint32_t *const *d_a, const siz
         }
         for (size_t i = 0; i < all.size(); i++) {
             const int k3 = k3s[i];
-            if (k3 >= 0 && (k3 >= g.r3_min_log || count3[k3] >= (1LL << (g.r3_min_log - k3)))) {
+            if (k3 >= 0 && (r3_alone(k3) || count3[k3] >= (1LL << (g.r3_min_log - k3)))) {
                 all[i].L = k3;
                 all[i].r3 = 1;
             }
@@ -2916,7 +2922,7 @@ int gbntt_server_submit(uint32_t *d_c, const uint32_t *d_a, size_t na, const uin
     r.item = BatchItem{d_c, d_a, d_b, na, nb};
     r.L = L;
     const int k3 = r3_log(na, nb);   // the single-product rule: the server cannot count future requests
-    if (k3 >= g.r3_min_log) {
+    if (r3_alone(k3)) {
         r.L = k3;
         r.r3 = 1;
     }

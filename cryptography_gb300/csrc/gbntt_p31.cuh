@@ -319,13 +319,12 @@ struct P31R3Args {
     uint32_t *spec[3];
     long long M, W;                     // 2^k, products (<= 65535)
     int shift;                          // 25 - k: w_N^j = rho^(j << shift)
-    int blocks;                         // blocks per prime
     const uint32_t *limbs;              // forward input of a single product, or of W products
     long long n_limbs;
     const uint32_t *const *limb_tab;
     const long long *len_tab;
     const uint32_t *rho[3];             // two-level tables of rho (order 3 2^25)
-    ShoupWord c[3], step[3];            // (om - om^2) / 2; w^G (forward) or w^-G (inverse), G = blocks x 256
+    ShoupWord c[3], step[3];            // (om - om^2) / 2; w (forward) or w^-1 (inverse)
 };
 cudaError_t launch_p31_radix3(bool inverse, const P31R3Args &a, cudaStream_t st);
 
