@@ -2295,6 +2295,40 @@ static int read_errors(unsigned *flags)
 // twist, the cyclic pass chain, the fused pointwise product and inverse,
 // then untwist + Garner to signed 256-bit coefficients (reference
 // pipeline_negacyclic, ntt/lib/main.hip:557-684).
+static int negacyclic_p31(uint64_t *d_out, const uint64_t *d_f, const uint64_t *d_g, int L, cudaStream_t st)
+{
+    // three products of 2^L points side by side (gbntt_p31_nega.cu)
+    const bool square = d_f == d_g;
+    const size_t N = (size_t)1 << L, stride = 3 * N / 2;   // 3 N 32-bit words per prime
+    uint64_t *specA = g.d_spec, *specB = g.d_spec + 3 * stride;
+    P31NegaArgs a;
+    memset(&a, 0, sizeof a);
+    a.coef[0] = d_f;
+    a.coef[1] = d_g;
+    a.shift = kP31MaxLog - 1 - L;
+    a.n = (long long)N;
+    a.out = d_out;
+    for (int k = 0; k < 3; k++) {
+        a.spec[0][k] = (uint32_t *)(specA + k * stride);
+        a.spec[1][k] = (uint32_t *)(specB + k * stride);
+        a.hi[k] = tw31(k, 0, 0);
+        a.lo[k] = tw31(k, 0, 1);
+    }
+    CK(launch_p31_nega_twist(square ? 1 : 2, a, st));
+    const P31Op ops[2] = {{specA, 3, nullptr, 0, nullptr, nullptr}, {specB, 3, nullptr, 0, nullptr, nullptr}};
+    int rc = p31_forward(ops, square ? 1 : 2, stride, L, st, true);
+    if (rc) return rc;
+    if ((rc = p31_inner(specA, specB, stride, L, 3, square ? P31_SQUARE : P31_OWN, false, nullptr, 0, st)) != GBNTT_OK)
+        return rc;
+    if ((rc = p31_inverse(specA, stride, L, 3, false, st)) != GBNTT_OK) return rc;
+    for (int k = 0; k < 3; k++) {
+        a.hi[k] = tw31(k, 1, 0);
+        a.lo[k] = tw31(k, 1, 1);
+    }
+    CK(launch_p31_nega_finish(a, st));
+    return GBNTT_OK;
+}
+
 static int negacyclic_dev(uint64_t *d_out, const uint64_t *d_f, const uint64_t *d_g, int L, cudaStream_t st)
 {
     if (!g.ready) { set_err("engine not initialised"); return GBNTT_ERR_NOT_INIT; }
@@ -2304,6 +2338,8 @@ static int negacyclic_dev(uint64_t *d_out, const uint64_t *d_f, const uint64_t *
         return GBNTT_ERR_ARG;
     }
     if (!d_out || !d_f || !d_g) { set_err("gbntt_negacyclic_mul_u64: null pointer"); return GBNTT_ERR_ARG; }
+    // (the 31-bit form's spectra take 72 N of the workspace's 48 n_max bytes)
+    if (use_p31(L + 1) && ((size_t)2 << L) <= g.n_max) return negacyclic_p31(d_out, d_f, d_g, L, st);
     const PrimeSet &ps = kSet3;
     const long long N = 1LL << L;
     uint64_t *specA = g.d_spec, *specB = g.d_spec + 3 * g.n_max;

@@ -366,6 +366,19 @@ cudaError_t launch_p31_block(int log_n, const P31BlockArgs &a, long long W, cuda
 // most 2^(log_n + 1) words) and returns their size.
 int p31_block_tables(int log_n, uint32_t *dst, uint64_t w, uint64_t p);
 
+// Negacyclic products of N = 2^L 64-bit coefficients, L < kP31MaxLog: three
+// products' spectra of N words, one after the other, per prime and operand.
+struct P31NegaArgs {
+    uint32_t *spec[2][3];
+    const uint64_t *coef[2];            // twist
+    const uint32_t *hi[3], *lo[3];      // two-level tables of w (order 2^25) or w^-1
+    int shift;                          // psi^i = w^(i << shift)
+    long long n;                        // N
+    uint64_t *out;                      // finish: 4 N words
+};
+cudaError_t launch_p31_nega_twist(int nops, const P31NegaArgs &a, cudaStream_t st);
+cudaError_t launch_p31_nega_finish(const P31NegaArgs &a, cudaStream_t st);
+
 cudaError_t launch_p31_pass(int log_l, int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st);
 cudaError_t launch_p31_contig_fwd(int log_l, const P31InnerArgs &a, cudaStream_t st);
 cudaError_t launch_p31_inner(int log_l, const P31InnerArgs &a, cudaStream_t st);

@@ -134,3 +134,34 @@ def test_knobs(knobs):
     r = subprocess.run([sys.executable, "-c", body], capture_output=True, text=True, timeout=600,
                        env=dict(os.environ, **knobs))
     assert r.returncode == 0 and "fine" in r.stdout, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("log_n", [5, 6, 8, 10, 11, 13, 17, 19, 22, 23])
+def test_negacyclic(engine, log_n):
+    # three products of 32-bit halves (gbntt_p31_nega.cu) against the three
+    # 64-bit primes: random and largest coefficients, squares
+    n = 1 << log_n
+    rng = np.random.default_rng(log_n)
+    f = rng.integers(0, 1 << 64, n, dtype=np.uint64)
+    g = rng.integers(0, 1 << 64, n, dtype=np.uint64)
+    full = np.full(n, 0xFFFFFFFFFFFFFFFF, dtype=np.uint64)
+    f[::7] = 0xFFFFFFFF00000000
+    bufs = []
+    for x in (f, g, full):
+        bufs.append(cudart.DeviceBuffer(8 * n))
+        bufs[-1].upload(x)
+    out = cudart.DeviceBuffer(32 * n)
+    for x, y in ((0, 1), (0, 0), (2, 2), (2, 1), (1, 2)):
+        got = []
+        for primes in (2, 3):
+            engine.set_prime_set(primes)
+            try:
+                engine.negacyclic_mul_device(out.ptr, bufs[x].ptr, bufs[y].ptr, log_n)
+                cudart.synchronize()
+                got.append(out.download(np.uint64, 4 * n))
+            finally:
+                engine.set_prime_set(2)
+        assert np.array_equal(*got), (x, y)
+    for b in bufs + [out]:
+        b.free()
+    assert engine.device_errors() == 0
