@@ -107,6 +107,7 @@ struct Engine {
     unsigned *d_ctl = nullptr;      // [0] ticket, [1] error, [2..] tile status
     size_t n_status = 0;
     uint32_t *d_io = nullptr;       // staging for host-pointer calls
+    uint32_t *h_short = nullptr;    // pinned: error word (16 bytes), then operands and product of a short host product
     size_t io_words = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;      // second prime's passes run here, overlapping the first's
@@ -377,12 +378,16 @@ static size_t workspace_bytes(int max_log)
     return spec + tw + ctl + io;
 }
 
+// Engine::h_short: 4 words, then n_a + n_b operand and as many product limbs.
+constexpr size_t kShortWords = 4 + 2 * (((size_t)1 << kP31BlockLog) + 1);
+
 static void invalidate_wave_graphs();
 
 static void free_all()
 {
     if (g.stream) cudaStreamSynchronize(g.stream);
     cudaFree(g.d_btab);
+    if (g.h_short) cudaFreeHost(g.h_short);
     if (g.h_btab) cudaFreeHost(g.h_btab);
     for (int i = 0; i < 2; i++) if (g.btab_ev[i]) cudaEventDestroy(g.btab_ev[i]);
     cudaFree(g.d_spec);
@@ -527,6 +532,12 @@ static int init_impl(int max_log)
     if (cudaMalloc(&g.d_btab, 2 * kBtabWords * sizeof(uint64_t)) != cudaSuccess ||
         cudaMallocHost(&g.h_btab, 2 * kBtabWords * sizeof(uint64_t)) != cudaSuccess) {
         set_err("gbntt_init: batch table allocation failed");
+        cudaGetLastError();
+        free_all();
+        return GBNTT_ERR_ALLOC;
+    }
+    if (cudaHostAlloc(&g.h_short, kShortWords * sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess) {
+        set_err("gbntt_init: pinned allocation failed");
         cudaGetLastError();
         free_all();
         return GBNTT_ERR_ALLOC;
@@ -2416,6 +2427,42 @@ static const void *managed_device_ptr(const void *p)
     return nullptr;
 }
 
+static int device_failure(unsigned flags)
+{
+    if (!flags) return GBNTT_OK;
+    set_err("device check failed (flags 0x%x): %s", flags,
+            (flags & ERR_GARNER_DIGIT) ? "CRT digit out of range" : "carry look-back wait gave up");
+    return GBNTT_ERR_DEVICE;
+}
+
+// A host product that runs in one CTA: the operands go into pinned memory
+// that the kernel reads over NVLink-C2C, and the product and the error bits
+// come back there, so the call is one launch and one wait instead of two
+// copies in, one out, and a copy and a clear of the error word
+// (96 x 64 limbs 43 -> 21 us).
+static int mul_host_short(uint32_t *c, const uint32_t *a, size_t na, const uint32_t *b, size_t nb, bool square)
+{
+    uint32_t *h = g.h_short;
+    h[0] = 0;
+    P31BlockArgs k;
+    memset(&k, 0, sizeof k);
+    uint32_t *ha = h + 4, *hb = square ? ha : ha + na, *hc = ha + na + nb;
+    memcpy(ha, a, na * 4);
+    if (!square) memcpy(hb, b, nb * 4);
+    k.limbs[0] = ha;
+    k.limbs[1] = hb;
+    k.n_limbs[0] = (long long)na;
+    k.n_limbs[1] = (long long)nb;
+    k.out = hc;
+    k.n_out = (long long)(na + nb);
+    k.sticky = g.d_ctl + 1;
+    const int rc = p31_block(k, choose_log(na, nb), 1, h, 8.0 * (double)(na + nb), g.stream);
+    if (rc) return rc;
+    CK(cudaStreamSynchronize(g.stream));
+    memcpy(c, hc, (na + nb) * 4);
+    return device_failure(h[0]);
+}
+
 static int mul_host(uint32_t *c, const uint32_t *a, size_t na, const uint32_t *b, size_t nb,
                     const uint32_t *dev_a, const uint32_t *dev_b)
 {
@@ -2427,6 +2474,8 @@ static int mul_host(uint32_t *c, const uint32_t *a, size_t na, const uint32_t *b
         return GBNTT_ERR_SIZE;
     }
     const bool square = (a == b && na == nb);
+    if (!dev_a && !dev_b && g.zero_copy && !g.prof && use_block(choose_log(na, nb)) && !r3_alone(r3_log(na, nb)))
+        return mul_host_short(c, a, na, b, nb, square);
     uint32_t *da = g.d_io, *db = g.d_io + na, *dc = g.d_io + na + (square ? 0 : nb);
     double t0 = g.prof ? now_ms() : 0;
     const uint32_t *ua = dev_a, *ub = dev_b;
@@ -2482,12 +2531,7 @@ static int mul_host(uint32_t *c, const uint32_t *a, size_t na, const uint32_t *b
     rc = read_errors(&flags);
     if (rc) return rc;
     if (g.prof) { double t = now_ms(); g.prof_ms[2] += t - t0; g.prof_calls++; }
-    if (flags) {
-        set_err("device check failed (flags 0x%x): %s", flags,
-                (flags & ERR_GARNER_DIGIT) ? "CRT digit out of range" : "carry look-back wait gave up");
-        return GBNTT_ERR_DEVICE;
-    }
-    return GBNTT_OK;
+    return device_failure(flags);
 }
 
 // Host-pointer packed product through the staging buffer.
@@ -2521,12 +2565,7 @@ static int mul_host64(uint64_t *c, const uint64_t *a, size_t na, const uint64_t 
     rc = read_errors(&flags);
     if (rc) return rc;
     if (g.prof) { double t = now_ms(); g.prof_ms[2] += t - t0; g.prof_calls++; }
-    if (flags) {
-        set_err("device check failed (flags 0x%x): %s", flags,
-                (flags & ERR_GARNER_DIGIT) ? "CRT digit out of range" : "carry look-back wait gave up");
-        return GBNTT_ERR_DEVICE;
-    }
-    return GBNTT_OK;
+    return device_failure(flags);
 }
 
 // ---- reference BigInt path -------------------------------------------------

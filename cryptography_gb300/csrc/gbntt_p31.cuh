@@ -360,6 +360,7 @@ struct P31BlockArgs {
     const uint32_t *tw[3][2];           // step tables per prime and direction (p31_block_tables)
     ShoupWord scale[3];                 // 2^32 / N
     unsigned *error;
+    unsigned *sticky;                   // or null: error bits moved from here to *error (one product)
 };
 cudaError_t launch_p31_block(int log_n, const P31BlockArgs &a, long long W, cudaStream_t st);
 // Fills the step tables of 2^log_n points for a root w of that order (at

@@ -264,6 +264,7 @@ __global__ void __launch_bounds__(BlockShape<LOG_N>::T) p31_block_kernel(const _
     __syncthreads();
     for (int j = tid; j < K * T; j += T)
         if (j < n_out) out[j] = sm[j];
+    if (a.sticky && tid == 0) err |= atomicExch(a.sticky, 0u);
     if (err) atomicOr(a.error, err);
 }
 
