@@ -90,9 +90,9 @@ constexpr P31Roots p31_roots()
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class Args>
 static inline cudaError_t launch_chained(void (*fn)(Args), dim3 grid, int threads, size_t smem, cudaStream_t st,
-                                         const Args &args)
+                                         const Args &args, int cluster = 1)
 {
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c = {};
@@ -102,6 +102,12 @@ static inline cudaError_t launch_chained(void (*fn)(Args), dim3 grid, int thread
     c.stream = st;
     c.attrs = at;
     c.numAttrs = 1;
+    if (cluster > 1) {
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = (unsigned)cluster;
+        at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+        c.numAttrs = 2;
+    }
     return cudaLaunchKernelEx(&c, fn, args);
 }
 
@@ -344,8 +350,8 @@ uint64_t p31_outer_root(int k);         // g of prime k
 uint64_t p31_outer_half(int k);         // g^(d / 2)
 cudaError_t p31_outer_init();
 
-// A whole product of up to 2^kP31BlockLog coefficients in one CTA (W of them:
-// the tables, one CTA each).
+// A whole product of up to 2^kP31BlockLog coefficients in one CTA or a cluster
+// of three (W of them: the tables).
 constexpr int kP31BlockLog = 12;
 struct P31BlockArgs {
     const uint32_t *limbs[2];

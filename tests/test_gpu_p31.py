@@ -94,6 +94,12 @@ def test_one_cta_waves(engine, L):
     A = [a, a[1:], d[:top // 2], d[1:top // 2]]
     _waves(engine, A, [b, b, a, a])
     _waves(engine, A[1:], [b] * 3)
+    # more products than take a cluster of CTAs each: the longest and the
+    # shortest of the length, so that every carry tile boundary is met
+    sizes = [(top // 2, top // 2 + 1 - i % 3) for i in range(57)] + [(top // 2 + 1, 1)] * 3
+    _waves(engine, [_rand(rng, n) for n, _ in sizes], [_rand(rng, n) for _, n in sizes])
+    full = np.full(top // 2, 0xFFFFFFFF, dtype=np.uint32)
+    _waves(engine, [full, full], [full, full.copy()])
     assert engine.device_errors() == 0
 
 
