@@ -1928,6 +1928,13 @@ static int batch_mul(uint32_t *const *d_c, const uint32_t *const *d_a, const siz
             }
             continue;
         }
+        if (!use_p31(r3_alone(r3_log(na[i], nb[i])) ? L - 2 : L) && p31_outer_blocks(na[i], nb[i])) {
+            // longer than a 31-bit transform: it fills the GPU by itself, and
+            // a wave of such products would run on q0 with p3 (a pair sharing
+            // its right operand 86 ms at 2^28 limbs, two products alone 68)
+            rc = mul_dev(d_c[i], d_a[i], na[i], d_b[i], nb[i], st);
+            continue;
+        }
         all.push_back({L, (long long)i, {d_c[i], d_a[i], d_b[i], na[i], nb[i]}});
     }
     if (rc == GBNTT_OK && split_words) {

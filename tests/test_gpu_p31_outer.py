@@ -70,3 +70,28 @@ def test_outer_stage_largest_coefficients(big, n):
     for x in (da, db, dc):
         x.free()
     assert big.device_errors() == 0
+
+
+def test_batch_of_long_products(big):
+    # a batch whose long products run one after the other beside a wave
+    sizes = [(M + 1, M), (M // 2, M), (1000, 900), (M + 1, M)]
+    A = [synth.operand(n, 50 + i) for i, (n, _) in enumerate(sizes)]
+    B = [synth.operand(n, 60 + i) for i, (_, n) in enumerate(sizes)]
+    da, db = [_device(x) for x in A], [_device(x) for x in B]
+    db[3] = db[0]   # the same right operand
+    dc = [cudart.DeviceBuffer(4 * (x + y)) for x, y in sizes]
+    one = cudart.DeviceBuffer(4 * (2 * M + 1))
+    big.batch_mul_device([c.ptr for c in dc], [x.ptr for x in da], [n for n, _ in sizes], [x.ptr for x in db],
+                         [n for _, n in sizes])
+    cudart.synchronize()
+    for i, (x, y) in enumerate(sizes):
+        big.set_prime_set(3)
+        try:
+            big.mul_device(one.ptr, da[i].ptr, x, db[i].ptr, y)
+            cudart.synchronize()
+        finally:
+            big.set_prime_set(2)
+        assert np.array_equal(dc[i].download(np.uint32, x + y), one.download(np.uint32, x + y)), i
+    for buf in {id(b): b for b in da + db + dc + [one]}.values():
+        buf.free()
+    assert big.device_errors() == 0
