@@ -1008,6 +1008,7 @@ static int p31_forward(const P31Op *ops, int nops, size_t stride, int L, cudaStr
         a.log_m = log_m;
         a.log_s = log_m - pl[i];
         a.log_prod = L;
+        a.by_table = i == 0;
         for (int k = 0; k < 3; k++) {
             a.ptw[k] = (const uint32_t *)pass_table(5 + k, 0, a.log_m, a.log_s, 0, 0, st);
             a.st[k] = g.d_st31 + ((size_t)k * 2 + 0) * kP31StepWords;
@@ -1103,6 +1104,7 @@ static int p31_inverse(uint64_t *spec, size_t stride, int L, long long W, bool r
         a.log_s = log_ms[i] - pl[i];
         a.ncols = W << (L - pl[i]);
         a.use_scale = i == 0;
+        a.by_table = i == 0;
         for (int k = 0; k < 3; k++) {
             a.data[0][k] = (uint32_t *)(spec + k * stride);
             a.st[k] = g.d_st31 + ((size_t)k * 2 + 1) * kP31StepWords;

@@ -303,6 +303,7 @@ struct P31PassArgs {
     int log_m, log_s;                   // sub-problem and column-stride logs
     int log_prod;                       // log2 of a product's coefficients (first pass)
     long long ncols;                    // columns per operand
+    int by_table;                       // the outermost pass: order the CTAs by their part of the table
 };
 
 struct P31InnerArgs {

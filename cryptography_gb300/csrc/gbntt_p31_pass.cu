@@ -24,6 +24,33 @@ constexpr long long kTwoColumns = 1LL << 20;
 // with one, 22.4 with four).
 constexpr long long kFourColumns = 1LL << 21;
 
+// First column, prime and operand of a CTA. Launches over many sub-problems
+// with a large table (by_table) take the CTAs that read the same part of the
+// table one after the other, so that it comes from HBM once: grid (prime and
+// operand, sub-problem, tile of columns); the others count tiles through.
+// Outermost passes over 16 sub-problems of 2^25 points: 6.51 -> 6.04 ms forward,
+// 3.09 -> 2.90 ms inverse; over 3 of 2^22 141 -> 129 and 74 -> 61 us.
+struct PassTile {
+    int k, op;
+    long long col0;
+};
+template <int G>
+__device__ __forceinline__ PassTile pass_tile_of(const P31PassArgs &a)
+{
+    if (a.by_table)
+        return {(int)(blockIdx.x % 3), (int)(blockIdx.x / 3),
+                ((long long)blockIdx.y << a.log_s) + (long long)blockIdx.z * G};
+    return {(int)(blockIdx.x % 3), (int)blockIdx.y, (long long)(blockIdx.x / 3) * G};
+}
+template <int G>
+dim3 pass_grid(P31PassArgs &a, int nops)
+{
+    const long long subs = a.ncols >> a.log_s, tiles = (1LL << a.log_s) / G;
+    a.by_table = a.by_table && subs * nops > 1 && subs <= 65535 && tiles <= 65535;
+    if (a.by_table) return dim3((unsigned)(3 * nops), (unsigned)subs, (unsigned)tiles);
+    return dim3((unsigned)(3 * (a.ncols / G)), (unsigned)nops);
+}
+
 // word at byte offset off of a base address
 template <class Word>
 __device__ __forceinline__ Word ld_off(const void *base, uint32_t off)
@@ -50,7 +77,7 @@ __device__ __forceinline__ uint32_t p31_tw(const P31PassArgs &a, int k, uint32_t
 // Shape of a strided tile with V adjacent columns per thread: GP threads
 // side by side, G = V GP columns. Exchange words are V residues wide, at
 // ka RS + b GP + gp.
-template <int LOG_L, int V, int DIR>
+template <int LOG_L, int V, int DIR, bool LIMBS = false>
 struct P31StridedShape {
     using S = P31Shape<LOG_L>;
     static constexpr int B = S::B;
@@ -61,7 +88,7 @@ struct P31StridedShape {
     static constexpr int LANES = 32 / V;   // threads served by one shared-memory access
     static constexpr int RS = B * GP + (GP < LANES ? GP : 0);
     static constexpr int MIN_BLOCKS = V == 1 ? (LOG_L >= 9 ? 3 : LOG_L == 5 ? 10 : 5)
-                                             : (LOG_L == 8 ? 3 + DIR : LOG_L == 5 ? 10 : 6);
+                                             : (LOG_L == 8 ? 3 + (DIR || LIMBS) : LOG_L == 5 ? 10 : 6);
 };
 template <int V>
 struct Residues;
@@ -86,17 +113,18 @@ struct Residues<2> {
 // 68%, issue 0.61, DRAM 51%). It wants twice the tiles to fill the GPU
 // (launch_l).
 template <int LOG_L, int DIR, bool LIMBS, int V>
-__global__ void __launch_bounds__(P31StridedShape<LOG_L, V, DIR>::T, P31StridedShape<LOG_L, V, DIR>::MIN_BLOCKS)
+__global__ void __launch_bounds__(P31StridedShape<LOG_L, V, DIR, LIMBS>::T, P31StridedShape<LOG_L, V, DIR, LIMBS>::MIN_BLOCKS)
 p31_pass_kernel(const __grid_constant__ P31PassArgs a)
 {
     using S = P31Shape<LOG_L>;
-    using H = P31StridedShape<LOG_L, V, DIR>;
+    using H = P31StridedShape<LOG_L, V, DIR, LIMBS>;
     using W = Residues<V>;
     typedef typename W::T Word;
     constexpr int A = S::A, B = S::B, GP = H::GP, RS = H::RS;
     __shared__ Word sm[A * RS];
-    const int k = blockIdx.x % 3, op = blockIdx.y;
-    const long long col0 = (long long)(blockIdx.x / 3) * H::G;
+    const PassTile at = pass_tile_of<H::G>(a);
+    const int k = at.k, op = at.op;
+    const long long col0 = at.col0;
     const uint32_t p = p31_prime(k), pinv = p31_inv(k);
     const int t = threadIdx.x, gp = t & (GP - 1), q = t >> H::LOG_GP;
     const int log_s = a.log_s;
@@ -261,8 +289,9 @@ __global__ void __launch_bounds__(512, 2) p31_pass9_kernel(const __grid_constant
 {
     constexpr int GP = 8, V = 4;
     extern __shared__ uint4 sm9[];
-    const int k = blockIdx.x % 3, op = blockIdx.y;
-    const long long col0 = (long long)(blockIdx.x / 3) * (V * GP);
+    const PassTile at = pass_tile_of<V * GP>(a);
+    const int k = at.k, op = at.op;
+    const long long col0 = at.col0;
     const uint32_t p = p31_prime(k), pinv = p31_inv(k);
     const int t = threadIdx.x, gp = t & (GP - 1), q = t >> 3;
     const int log_s = a.log_s;
@@ -394,7 +423,7 @@ __global__ void __launch_bounds__(512, 2) p31_pass9_kernel(const __grid_constant
         st_off<uint4>(data, out0 + i * step, make_uint4(x[0][i], x[1][i], x[2][i], x[3][i]));
 }
 
-cudaError_t launch_9(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
+cudaError_t launch_9(int dir, bool limbs, int nops, P31PassArgs &a, cudaStream_t st)
 {
     constexpr size_t smem = 64 * 64 * sizeof(uint4);
     static const cudaError_t attr[3] = {
@@ -406,14 +435,14 @@ cudaError_t launch_9(int dir, bool limbs, int nops, const P31PassArgs &a, cudaSt
     return launch_chained(dir == 1 ? p31_pass9_kernel<1, false>
                           : limbs  ? p31_pass9_kernel<0, true>
                                    : p31_pass9_kernel<0, false>,
-                          dim3((unsigned)(3 * (a.ncols / 32)), (unsigned)nops), 512, smem, st, a);
+                          pass_grid<32>(a, nops), 512, smem, st, a);
 }
 
 template <int LOG_L, int V>
-cudaError_t launch_v(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
+cudaError_t launch_v(int dir, bool limbs, int nops, P31PassArgs &a, cudaStream_t st)
 {
     using H = P31StridedShape<LOG_L, V, 0>;
-    const dim3 grid((unsigned)(3 * (a.ncols / H::G)), (unsigned)nops);
+    const dim3 grid = pass_grid<H::G>(a, nops);
     return launch_chained(dir == 1 ? p31_pass_kernel<LOG_L, 1, false, V>
                           : limbs  ? p31_pass_kernel<LOG_L, 0, true, V>
                                    : p31_pass_kernel<LOG_L, 0, false, V>,
@@ -421,7 +450,7 @@ cudaError_t launch_v(int dir, bool limbs, int nops, const P31PassArgs &a, cudaSt
 }
 
 template <int LOG_L>
-cudaError_t launch_l(int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
+cudaError_t launch_l(int dir, bool limbs, int nops, P31PassArgs &a, cudaStream_t st)
 {
     if constexpr (LOG_L <= 8) {   // (more points leave too few warps: 32 or more residues per column in registers)
         if ((a.ncols << LOG_L) * nops >= kTwoColumns) return launch_v<LOG_L, 2>(dir, limbs, nops, a, st);
@@ -446,8 +475,9 @@ __global__ void p31_table_kernel(int k, uint32_t *table, const uint32_t *hi, con
 
 }  // namespace
 
-cudaError_t launch_p31_pass(int log_l, int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st)
+cudaError_t launch_p31_pass(int log_l, int dir, bool limbs, int nops, const P31PassArgs &args, cudaStream_t st)
 {
+    P31PassArgs a = args;
     switch (log_l) {
     case 5: return launch_l<5>(dir, limbs, nops, a, st);
     case 6: return launch_l<6>(dir, limbs, nops, a, st);
