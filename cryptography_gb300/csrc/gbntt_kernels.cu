@@ -405,12 +405,15 @@ __global__ void __launch_bounds__(kCarryThreads, GBNTT_CARRY_MIN_BLOCKS) garner_
 // shared memory it executed 112 instructions per coefficient: 138 us at 2^25
 // coefficients against 115 (4.7 TB/s) here, 16.3 against 14.3 at 2^21. Five
 // resident CTAs: 4 take 127 us, 6 123.
+// Limbs leave a warp as two runs of 512 bytes: stored straight from the
+// registers, 16 of every 32 bytes per instruction, a product in pinned host
+// memory (2^28 x 2^28 limbs, ntt_bigint_mul) took 60.6 ms against 49.9.
 template <bool BATCH>
 __global__ void __launch_bounds__(kCarryThreads, 5) garner_carry31_kernel(CarryArgs a)
 {
     constexpr int T = kCarryThreads, K = kCarryPerThread, TILE = kCarryTile;
     __shared__ uint32_t s_edge[T / 32 + 1][3];
-    __shared__ uint32_t s_out[TILE + TILE / 32];
+    __shared__ __align__(16) uint32_t s_out[TILE + TILE / 32];
     __shared__ unsigned s_warp[T / 32];
     __shared__ unsigned s_tile, s_cin;
     __shared__ long long s_prod;
@@ -509,9 +512,13 @@ __global__ void __launch_bounds__(kCarryThreads, 5) garner_carry31_kernel(CarryA
         o[k] = (uint32_t)x;
     }
     if (((uintptr_t)a.out & 15) == 0 && base + TILE <= a.n_out) {
-        uint4 *q = (uint4 *)(a.out + j0);
-        q[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        q[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        uint4 *row = (uint4 *)s_out + warp * 64, *q = (uint4 *)(a.out + base) + warp * 64;
+        auto sw = [](int c) { return c ^ ((c >> 3) & 1); };   // (bank-conflict free both ways)
+        row[sw(2 * lane)] = make_uint4(o[0], o[1], o[2], o[3]);
+        row[sw(2 * lane + 1)] = make_uint4(o[4], o[5], o[6], o[7]);
+        __syncwarp();
+        q[lane] = row[sw(lane)];
+        q[32 + lane] = row[sw(32 + lane)];
     } else {
 #pragma unroll
         for (int k = 0; k < K; k++) s_out[spad(tid * K + k)] = o[k];
