@@ -370,13 +370,20 @@ constexpr size_t kRecipHostLimbs = 64;
 // warp per piece then carries the column blocks into limbs, subtracts and
 // corrects (warp_resolve, warp_addsub).
 // ---------------------------------------------------------------------------
-constexpr int kDecThreads = 128;
-constexpr int kDecWarps = kDecThreads / 32;
+// Threads per CTA: the column sums bind the kernel (level 11 alone is 3.7 M
+// limb products), so a CTA that has an SM to itself takes enough warps to
+// fill its multiply pipes: 1 piece of level 11 0.61 ms with 128 threads, 0.42
+// with 512, 0.41 with 1024 (to_decimal of 3000 limbs 0.90 -> 0.70 ms, of
+// 250007, 66 pieces, 3.97 -> 3.78). With more CTAs than SMs fewer threads
+// balance better: 183 pieces 6.27 ms with 128 threads in to_decimal, 5.97 with
+// 256, 6.2 with 512; 523 pieces 13.4, 13.5 and 14.
+constexpr int kDecWide = 512;        // at most one CTA per SM
+constexpr int kDecThreads = 256;
 constexpr int kDecCols = 5;          // product columns per thread item; odd, so that the
                                      // lanes' operand reads (stride kDecCols) hit distinct banks
 constexpr int kDecPad = kDecCols;    // zero limbs on either side of d_j and mu_j in the table
 constexpr int kDecMaxTop = 12;       // highest level whose constants exist
-constexpr int kDecLeafLog = 7;       // at most 2^7 = kDecThreads printed pieces per CTA
+constexpr int kDecLeafLog = 7;       // at most 2^7 printed pieces per CTA, one thread each
 constexpr unsigned ERR_E_DECIMAL = 8u;   // a split's quotient or correction out of bounds
 
 struct DecLevel {
@@ -545,7 +552,8 @@ __device__ __forceinline__ uint32_t warp_addsub(uint32_t *dst, const uint32_t *x
     return cin;
 }
 
-__global__ void __launch_bounds__(kDecThreads) dec_block_kernel(const DecArgs A)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) dec_block_kernel(const DecArgs A)
 {
     extern __shared__ uint32_t dsm[];
     uint32_t *cur = dsm, *nxt = dsm + A.buf_limbs;
@@ -556,7 +564,7 @@ __global__ void __launch_bounds__(kDecThreads) dec_block_kernel(const DecArgs A)
     {
         const int S = A.lv[A.top].stride;
         const uint32_t *src = A.pieces + piece * S;
-        for (int i = tid; i < S; i += kDecThreads) cur[i] = src[i];
+        for (int i = tid; i < S; i += THREADS) cur[i] = src[i];
     }
     __syncthreads();
     for (int j = A.top; j >= A.low; j--) {
@@ -565,13 +573,13 @@ __global__ void __launch_bounds__(kDecThreads) dec_block_kernel(const DecArgs A)
         const int m = 1 << (A.top - j);
         const uint32_t *d = A.ctab + lv.off_d, *mu = A.ctab + lv.off_mu;
         // quotient estimate: columns n - 1 .. of floor(x / beta^(n-1)) mu
-        for (int it = tid; it < m * nb; it += kDecThreads) {
+        for (int it = tid; it < m * nb; it += THREADS) {
             const int p = it / nb, t = it - p * nb;
             dec_colblock(cur + p * S + (n - 1), n + 1, mu, n + 1, n - 1 + t * kDecCols, BL + (size_t)it * kDecCols,
                          BK + 2 * (size_t)it);
         }
         __syncthreads();
-        for (int p = warp; p < m; p += kDecWarps) {   // one warp per piece
+        for (int p = warp; p < m; p += THREADS / 32) {   // one warp per piece
             uint32_t *L = BL + (size_t)p * nb * kDecCols;
             const uint64_t over = warp_resolve(L, BK + 2 * (size_t)p * nb, nb, lane);
             uint32_t *q = nxt + (2 * p) * Sc;   // limb u of q' is column n + 1 + u
@@ -581,13 +589,13 @@ __global__ void __launch_bounds__(kDecThreads) dec_block_kernel(const DecArgs A)
         __syncthreads();
         // r' = x - q' d_j modulo beta^(n+1): columns 0 .. n of q' d_j
         const int nbr = (n + 1 + kDecCols - 1) / kDecCols;
-        for (int it = tid; it < m * nbr; it += kDecThreads) {
+        for (int it = tid; it < m * nbr; it += THREADS) {
             const int p = it / nbr, t = it - p * nbr;
             const int o = p * nb + t;
             dec_colblock(nxt + (2 * p) * Sc, n, d, n, t * kDecCols, BL + (size_t)o * kDecCols, BK + 2 * (size_t)o);
         }
         __syncthreads();
-        for (int p = warp; p < m; p += kDecWarps) {
+        for (int p = warp; p < m; p += THREADS / 32) {
             uint32_t *L = BL + (size_t)p * nb * kDecCols;
             warp_resolve(L, BK + 2 * (size_t)p * nb, nbr, lane);
             const uint32_t *x = cur + p * S;
@@ -623,7 +631,7 @@ __global__ void __launch_bounds__(kDecThreads) dec_block_kernel(const DecArgs A)
     // division by 10^9 in place
     const int groups = 1 << A.low, npr = 1 << (A.top - A.low + 1), W = A.leaf_stride;
     char *out = A.digits + piece * (9LL << (A.top + 1));
-    for (int p = tid; p < npr; p += kDecThreads) {
+    for (int p = tid; p < npr; p += THREADS) {
         uint32_t *x = cur + p * W;
         int nl = W;
         while (nl > 0 && x[nl - 1] == 0) nl--;
@@ -1795,16 +1803,21 @@ struct Pipe {
             a.buf_limbs = (int)buf;
             a.blk_items = (int)blk;
             const size_t smem = (size_t)(2 * buf + blk * (kDecCols + 2)) * sizeof(uint32_t);
+            const long long ncta = (1LL << (J - top)) - a.first;
+            int dev = 0, sms = 0;
+            ECK(cudaGetDevice(&dev));
+            ECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            const bool wide = ncta <= sms;
+            const int threads = wide ? kDecWide : kDecThreads;
+            void (*const kernel)(const DecArgs) = wide ? dec_block_kernel<kDecWide> : dec_block_kernel<kDecThreads>;
             if (smem > 48 * 1024) {
-                int dev = 0, cap = 0;
-                ECK(cudaGetDevice(&dev));
+                int cap = 0;
                 ECK(cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
                 if (smem > (size_t)cap) efail(GBNTT_ERR_SIZE, "decimal block of level %d needs %zu bytes of shared "
                                               "memory (%d available)", top, smem, cap);
-                ECK(cudaFuncSetAttribute(dec_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                ECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             }
-            const long long ncta = (1LL << (J - top)) - a.first;
-            dec_block_kernel<<<(unsigned)ncta, kDecThreads, smem, g_st>>>(a);
+            kernel<<<(unsigned)ncta, (unsigned)threads, smem, g_st>>>(a);
             ECK(cudaGetLastError());
             if (prof) {
                 sync();
