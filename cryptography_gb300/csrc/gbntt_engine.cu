@@ -4,8 +4,8 @@
 // ntt/lib/arith/ntt_mul.hip:312-347) guarded by a mutex, so concurrent host
 // callers serialise here instead of relying on the caller's lock
 // (ntt/lib/arith/multiply.c:27). Unlike the reference, the transform length
-// is chosen per call (the smallest power of two >= n_a + n_b - 1, at least
-// 32) instead of always the init-time maximum (ntt_mul.hip:1001-1002), and
+// is chosen per call (at least 32; a power of two, 3 2^k, or above 2^25 a
+// multiple of 2^25) instead of always the init-time maximum (ntt_mul.hip:1001-1002), and
 // twiddle tables are two-level (2 x 2^15 entries per prime and direction,
 // L2-resident) instead of O(N) host-built tables (ntt_mul.hip:189-308).
 #include <cuda_runtime.h>
@@ -53,10 +53,11 @@ static const uint64_t kGen[3] = {7, 10, 19};   // reference PRIM_ROOT[0, 2, 3]
 static const uint64_t kGen3 = 5;                 // primitive root of p3 = 3 * 2^30 + 1
 static uint32_t h_mont3(uint64_t x) { return (uint32_t)(((x % kP3) << 32) % kP3); }   // x 2^32 mod p3
 
-// Prime sets. Two primes (q0 with 64-bit residues, p3 with 32-bit residues)
-// carry every product of 32-bit coefficients: q0 p3 ~ 2^95.6 exceeds the
-// largest coefficient (< 2^93). The reference's three 64-bit primes stay
-// for 64-bit coefficients (packed mode, bound 2^158) and on request.
+// Prime sets of 64-bit words. Two primes (q0 with 64-bit residues, p3 with
+// 32-bit residues) carry the products of 32-bit coefficients that the three
+// 31-bit primes (gbntt_p31.cuh, use_p31) don't take: q0 p3 ~ 2^95.6 exceeds
+// the largest coefficient (< 2^93). The reference's three 64-bit primes stay
+// for 64-bit coefficients (long packed products, bound 2^158) and on request.
 struct PrimeSet {
     int n;
     int pi[3];
@@ -78,7 +79,7 @@ struct Engine {
     uint32_t *d_tw3 = nullptr;      // p3: [dir][hi|lo][2^15]
     uint64_t *d_st1 = nullptr;      // step-1 tables: [table slot 0..3][dir][kStep1Words]
     uint32_t *d_st13 = nullptr;     // p3's: [dir][kStep1Words]
-    int prime_set = 2;              // primes used for 32-bit coefficients: 2 or 3
+    int prime_set = 2;              // 32-bit coefficients: 2 (31-bit primes, or q0 with p3) or 3 (64-bit primes)
     bool q0_lazy = false;           // two-prime set: q0 as prime 4 (lazy normal form) or 0 (Montgomery)
     bool overlap = true;            // two-prime set: second prime's passes on stream2
     bool zero_copy = true;          // host-pointer calls: kernels read/write pinned host memory directly
@@ -102,7 +103,7 @@ struct Engine {
     ShoupWord r3c31[3] = {};        // (om - om^2) / 2 per prime
     uint64_t rho31[3] = {};         // rho (order 3 2^25) per prime
     bool batch_split = true;        // uneven batch products split into chunk products
-    int split_ratio_log = 3;        // ... when the longer operand is >= 2^this x the shorter
+    int split_ratio_log = 4;        // ... when the longer operand is >= 2^this x the shorter
     uint64_t garner2[2] = {0, 0};   // two-prime Garner constants (p3 Montgomery multipliers)
     unsigned *d_ctl = nullptr;      // [0] ticket, [1] error, [2..] tile status
     size_t n_status = 0;
@@ -1167,12 +1168,31 @@ static int p31_outer(const P31Op &op, size_t stride, int R, bool inverse, cudaSt
     return GBNTT_OK;
 }
 
+// Host -> device copy of the second operand, issued once the first operand's
+// first pass or outer stage has read its limbs (both share the host link).
+struct StageJob {
+    uint32_t *dst = nullptr;
+    const uint32_t *src = nullptr;   // device-mapped pinned memory, or a host pointer
+    size_t n = 0;
+    bool mapped = false;
+};
+
+// Copies an operand on the copy stream, ev_b when done.
+static int copy_operand(const StageJob &j)
+{
+    if (j.mapped) CK(launch_copy_words(j.dst, j.src, (long long)j.n, g.sms / 2, g.cstream));
+    else CK(cudaMemcpyAsync(j.dst, j.src, j.n * 4, cudaMemcpyHostToDevice, g.cstream));
+    CK(cudaEventRecord(g.ev_b, g.cstream));
+    return GBNTT_OK;
+}
+
 // Residues of W products a b in A's spectra, ready for the carry kernel:
 // transforms of R 2^L points, R = 1, 3 (the radix-3 stage) or, with W = 1
-// and L = 25, up to kP31MaxOuter (the outer stage). b_ready (optional): an
-// event that B's limbs wait for; A is transformed first then.
+// and L = 25, up to kP31MaxOuter (the outer stage). copy_b (optional): B's
+// limbs are copied on the copy stream once A's outer stage, if it has one, has
+// read A, which may be in host memory; A is transformed meanwhile.
 static int p31_products(const P31Op &A, const P31Op &B, size_t stride, int L, int R, P31Right right, unsigned *ctl,
-                        long long nzero, cudaStream_t st, cudaEvent_t b_ready = nullptr)
+                        long long nzero, cudaStream_t st, const StageJob *copy_b = nullptr)
 {
     const P31Op in[2] = {A, B};
     const int nops = right == P31_SQUARE ? 1 : 2;
@@ -1182,11 +1202,18 @@ static int p31_products(const P31Op &A, const P31Op &B, size_t stride, int L, in
         return R == 3 ? p31_radix3(in[o], stride, L, inverse, st) : p31_outer(in[o], stride, R, inverse, st);
     };
     for (int o = 0; o < nops; o++) sub[o].W *= R;
-    if (b_ready && nops == 2) {
+    if (copy_b && nops == 2) {
         for (int o = 0; o < 2; o++) {
-            if (o == 1) CK(cudaStreamWaitEvent(st, b_ready, 0));
+            if (o == 1) CK(cudaStreamWaitEvent(st, g.ev_b, 0));
             if (R > 1 && (rc = stage(o, false)) != GBNTT_OK) return rc;
+            if (o == 0) {
+                CK(cudaEventRecord(g.ev_a, st));
+                CK(cudaStreamWaitEvent(g.cstream, g.ev_a, 0));
+                if (copy_b->mapped && (rc = copy_operand(*copy_b)) != GBNTT_OK) return rc;
+            }
             if ((rc = p31_forward(sub + o, 1, stride, L, st, R > 1)) != GBNTT_OK) return rc;
+            // (a copy from pageable memory keeps the calling thread)
+            if (o == 0 && !copy_b->mapped && (rc = copy_operand(*copy_b)) != GBNTT_OK) return rc;
         }
     } else {
         for (int o = 0; R > 1 && o < nops; o++)
@@ -1256,17 +1283,6 @@ static int carry(const PrimeSet &ps, uint32_t *d_c, size_t n_out, const uint64_t
     rec_end(st);
     return GBNTT_OK;
 }
-
-// b_ready (optional): an event the second operand's transform waits for
-// (its host -> device copy on another stream).
-// Host -> device copy of the second operand, issued by mul_dev once the
-// first operand's first pass has read its limbs (both share the host link).
-struct StageJob {
-    uint32_t *dst = nullptr;
-    const uint32_t *src = nullptr;   // device-mapped pinned memory, or a host pointer
-    size_t n = 0;
-    bool mapped = false;
-};
 
 // Sub-transform log k of a length-3 2^k transform for an n_a x n_b product
 // when that is shorter than the power-of-two one (the product needs at most
@@ -1400,33 +1416,33 @@ static int r3_residues(const uint32_t *d_a, size_t na, const uint32_t *d_b, size
     return join_aux(st, aux);
 }
 
+// Points from which the copy of a second operand in host memory runs beside
+// the first one's transform, which then has launches of its own, instead of
+// before both: 2^20 x 2^20 limbs 212 -> 204 us from pinned memory and 246 ->
+// 229 from pageable, 2^24 x 2^24 2.82 -> 2.67 and 3.09 -> 2.75 ms; 2^19 x 2^19
+// 124.6 -> 127 and 153 -> 149 us, 2^17 x 2^17 60 -> 62 and 88 -> 88.
+constexpr size_t kCopyBeside = (size_t)1 << 21;
+
 // c = a b on the 31-bit prime set, transforms of R 2^L points. stage_a,
-// stage_b: operands in host memory, copied first; with the outer stage the
-// copy of B runs while A is transformed.
+// stage_b: operands in host memory, copied first, B from kCopyBeside points on
+// while A is transformed. With the outer stage A is not copied but read over
+// the link by that stage, which reads each limb once (2^28 limbs: 5 ms for
+// both, against 5 and 3).
 static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint32_t *d_b, size_t nb, int L, int R,
                        cudaStream_t st, const StageJob *stage_b, uint32_t *stage_a)
 {
     const bool square = (d_a == d_b && na == nb);
-    if (stage_a) {
+    const bool outer = L == kP31MaxLog && R > 1 && R != 3;   // (R = 3 is the radix-3 stage)
+    if (stage_a && !outer) {
         CK(launch_copy_words(stage_a, d_a, (long long)na, g.sms * 4, st));
         d_a = stage_a;
         if (square) d_b = stage_a;
     }
-    cudaEvent_t b_ready = nullptr;
+    const StageJob *copy_b = nullptr;
     if (stage_b && !square) {
-        cudaStream_t cs = st;
-        if (L == kP31MaxLog && R > 1) {   // after A's copy, which shares the host link
-            CK(cudaEventRecord(g.ev_a, st));
-            CK(cudaStreamWaitEvent(g.cstream, g.ev_a, 0));
-            cs = g.cstream;
-        }
-        if (stage_b->mapped)
-            CK(launch_copy_words(stage_b->dst, stage_b->src, (long long)stage_b->n, cs == st ? g.sms * 4 : g.sms / 2, cs));
-        else CK(cudaMemcpyAsync(stage_b->dst, stage_b->src, stage_b->n * 4, cudaMemcpyHostToDevice, cs));
-        if (cs != st) {
-            CK(cudaEventRecord(g.ev_b, cs));
-            b_ready = g.ev_b;
-        }
+        if (((size_t)R << L) >= kCopyBeside) copy_b = stage_b;
+        else if (stage_b->mapped) CK(launch_copy_words(stage_b->dst, stage_b->src, (long long)stage_b->n, g.sms * 4, st));
+        else CK(cudaMemcpyAsync(stage_b->dst, stage_b->src, stage_b->n * 4, cudaMemcpyHostToDevice, st));
     }
     if (R == 1 && use_block(L)) {
         P31BlockArgs a;
@@ -1441,7 +1457,7 @@ static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint
     }
     const P31Op A{g.d_spec, 1, d_a, na, nullptr, nullptr}, B{g.d_spec + 3 * g.n_max, 1, d_b, nb, nullptr, nullptr};
     const int rc = p31_products(A, B, g.n_max, L, R, square ? P31_SQUARE : P31_OWN, g.d_ctl,
-                                carry_tiles((long long)(na + nb)), st, b_ready);
+                                carry_tiles((long long)(na + nb)), st, copy_b);
     if (rc) return rc;
     return carry(kSet31, d_c, na + nb, g.d_spec, g.n_max, L, st, (long long)R << L, (long long)std::min(na, nb));
 }
@@ -1839,8 +1855,8 @@ static int g_batch_slot = 0;
 
 // Uneven products in a batch: a product whose longer operand (nB limbs) is
 // at least 2^split_ratio_log times its shorter one (nS limbs, at least
-// kSplitMinShort) and whose transform would be longer than the chunks' is
-// split into chunk products: the longer operand in
+// kSplitMinShort) and whose transform would be longer than the chunks' and
+// than one CTA's (use_block) is split into chunk products: the longer operand in
 // chunks of 2^ls - nS + 1 limbs (2^ls = 4 x the power of two >= nS), each
 // multiplied by the shorter operand at transform length 2^ls, so a
 // 2^21 x 2^13 product becomes 86 products of 2^15 points (the shorter
@@ -2502,11 +2518,12 @@ static int mul_host(uint32_t *c, const uint32_t *a, size_t na, const uint32_t *b
     const uint32_t *ua = dev_a, *ub = dev_b;
     // Zero copy: a pinned result is written by the carry kernel over
     // NVLink-C2C. Pinned operands: without stage_inputs the first forward
-    // passes of both primes read them in place (twice over C2C). With it
-    // (default) A's first q0 pass reads A over C2C once and leaves a copy in
-    // HBM for p3's first pass, and B is pulled into HBM by a copy kernel on
-    // the copy stream while A is being transformed. Pageable operands go
-    // through cudaMemcpyAsync.
+    // passes read them in place, each limb once per prime (the outer stage:
+    // once). With it (default) each limb crosses the link once: A is read in
+    // place by the outer stage, or copied first, or (q0 with p3) copied by its
+    // first q0 pass for p3's, and B is pulled into HBM by a copy kernel, for
+    // long products on the copy stream while A is being transformed. Pageable
+    // operands go through cudaMemcpyAsync.
     if (!ua && g.zero_copy && !g.stage_inputs) ua = (const uint32_t *)pinned_device_ptr(a);
     if (!ub && !square && g.zero_copy && !g.stage_inputs) ub = (const uint32_t *)pinned_device_ptr(b);
     uint32_t *uc = g.zero_copy ? (uint32_t *)pinned_device_ptr(c) : nullptr;
