@@ -2,12 +2,12 @@
 """Benchmark of the CRT-NTT big-integer multiply on one GB300.
 
 Workload (default): one multiply of two seeded uniform-random operands of
-2^28 32-bit limbs (1 GiB each), transform length N = 2^29 per prime over two
-primes: q0 = 2^64 - 2^32 + 1 (uint64 residues) and p3 = 3 * 2^30 + 1
-(uint32 residues), whose product exceeds every coefficient of the product
+2^28 32-bit limbs (1 GiB each), transform length N = 2^29 per prime over
+three 31-bit primes (uint32 residues, 64-bit products), whose product exceeds
+every coefficient of the product
 (the reference's three 64-bit primes 2^64 - 2^b + 1, b = 32, 34, 40, are
-timed beside it). A step is one full multiply (decomposition, 2 x 2 forward
-transforms, pointwise product, 2 inverse transforms, Garner + carry).
+timed beside it). A step is one full multiply (decomposition, 3 x 2 forward
+transforms, pointwise product, 3 inverse transforms, Garner + carry).
 Inputs (2 x 1 GiB) and the 12 GiB of spectra are far larger than the 129 MB
 L2, so no L2 flush is needed between steps.
 
@@ -633,7 +633,7 @@ def run_gpu(args, dist):
         flags |= g.device_errors()
         three = {"ms": tms, "steps": args.three_prime_steps,
                  "primes": "2^64-2^b+1, b = 32, 34, 40 (the reference's set; 64-bit residues)",
-                 "note": "same product, same transform length; the headline uses two primes"}
+                 "note": "same product, same transform length; the headline uses three 31-bit primes"}
 
     # squaring of the same operand (one forward transform), reported apart
     square = small = None
@@ -683,7 +683,7 @@ def run_gpu(args, dist):
     if radix3:
         flags |= radix3["device_error_flags"]
 
-    # packed mode (one 64-bit limb per coefficient, transform length 2^lg)
+    # packed mode (the same integers as 64-bit limbs)
     packed = None
     if not args.no_packed:
         def step64():
@@ -704,8 +704,9 @@ def run_gpu(args, dist):
         bmp = 10 * 3 * (1 << lg) * 8 + 8 * (2 * n)
         packed = {"ms": pms, "transform_log": lg, "bytes_model": bmp,
                   "multiply_roofline_frac": bmp / (pms * 1e-3) / 1e9 / peaks()[0],
-                  "note": "same integers as 2^%d 64-bit limbs, one coefficient per limb (reference granularity); "
-                          "not the headline configuration" % (lg - 1)}
+                  "note": "gbntt_mul_u64: same integers as 2^%d 64-bit limbs, which run as 32-bit limbs where the "
+                          "31-bit primes take them; bytes_model is that of one coefficient per limb over "
+                          "three 64-bit primes" % (lg - 1)}
 
     negacyclic = None
     if not args.no_negacyclic and dist.rank == 0:
@@ -743,7 +744,7 @@ def run_gpu(args, dist):
     for d in by_kind.values():
         d["share"] = d["ms"] / tot
         d["GBps"] = d["bytes"] / (d["ms"] * 1e-3) / 1e9 if d["ms"] > 0 else None
-    pass_kinds = [k for k in by_kind if "pass" in k]
+    pass_kinds = [k for k in by_kind if "pass" in k or "outer" in k]
     pass_ms = sum(by_kind[k]["ms"] for k in pass_kinds)
     pass_bytes = sum(by_kind[k]["bytes"] for k in pass_kinds)
     pass_launches = sum(by_kind[k]["launches"] for k in pass_kinds)
@@ -754,7 +755,7 @@ def run_gpu(args, dist):
     if os.path.exists(tp):
         try:
             tj = json.load(open(tp))
-            traffic = tj.get("ntt_pass_kernel_bytes_per_launch" if g.prime_set() == 2 else
+            traffic = tj.get("p31_pass_bytes_per_launch" if g.prime_set() == 2 else
                              "three_prime_64bit_bytes_per_launch")
         except (ValueError, OSError):
             traffic = None
@@ -763,17 +764,18 @@ def run_gpu(args, dist):
     if os.path.exists(ip) and g.prime_set() == 2:
         try:
             ij = json.load(open(ip))
-            scale = float(1 << (lg + 1)) / float(1 << 27)   # the capture's transform length is 2^27
-            inst = ij["multiply_2pow27_warp_instructions"] * scale
-            alu = ij["multiply_2pow27_alu_warp_instructions"] * scale
+            scale = float(1 << (lg + 1)) / float(1 << 29)   # the capture's transform length is 2^29
+            inst = ij["multiply_2pow29_warp_instructions"] * scale
+            alu = ij["multiply_2pow29_alu_warp_instructions"] * scale
+            fma = ij["multiply_2pow29_fmaheavy_warp_instructions"] * scale
             sms = cudart.sm_count()
             sm_hz = float((clk or {}).get("sm_mhz") or 2070.0) * 1e6   # SM clock sampled in the timed region
             cap = sms * 4 * sm_hz * ms * 1e-3          # warp-instruction issue slots in one multiply
             issue = {"bound": "integer issue", "instructions_per_multiply": inst,
                      "achieved": inst / (ms * 1e-3), "peak": sms * 4 * sm_hz, "unit": "warp instructions/s",
-                     "frac": inst / cap, "alu_pipe_frac": 2.0 * alu / cap,
+                     "frac": inst / cap, "alu_pipe_frac": 2.0 * alu / cap, "fmaheavy_pipe_frac": 2.0 * fma / cap,
                      "sm_mhz": sm_hz / 1e6, "source": "profiles/ncu_issue.json (ncu instruction counts of one "
-                                                    "2^27-point multiply, scaled to this transform length)"}
+                                                    "2^29-point multiply, scaled to this transform length)"}
         except (ValueError, OSError, KeyError):
             issue = None
     bm = bytes_model(lg)
@@ -828,19 +830,19 @@ def run_gpu(args, dist):
     line = {
         "metric": METRIC, "value": ms, "unit": UNIT, "n_gpus": dist.world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": False, "scaling": "weak",
-        "vs_baseline": None, "dtype": "u64",
+        "vs_baseline": None, "dtype": "u32" if g.prime_set() == 2 else "u64",
         "data": "synthetic (seeded splitmix64 limbs; inputs resident in HBM)",
         "config": {"workload": "multiply 2^%d x 2^%d 32-bit limbs, NTT length 2^%d per prime, bit-exact"
                                % (lg, lg, lg + 1),
-                   "primes": "q0 = 2^64-2^32+1 (uint64 residues) and p3 = 3*2^30+1 (uint32 residues); CRT "
-                             "modulus 2^95.6 > largest coefficient 2^92; the reference's three 64-bit primes "
+                   "primes": "15*2^27+1, 27*2^26+1, 63*2^25+1 (uint32 residues); CRT "
+                             "modulus 2^92.6 > largest coefficient 2^92; the reference's three 64-bit primes "
                              "are timed in three_prime_64bit" if g.prime_set() == 2 else
                              "2^64-2^b+1, b = 32, 34, 40 (uint64 residues)",
-                   "operand_limbs": n, "transform_log": lg + 1, "passes": g.plan(lg + 1),
-                   "l2_policy": "inputs and 24 GiB spectra >> 129 MB L2; no flush", "parallelism": "replicas"},
+                   "operand_limbs": n, "transform_log": lg + 1, "passes": [log_l for kind, log_l, _, _ in recs if kind not in ("garner_carry", "carry")],
+                   "l2_policy": "inputs and 12 GiB spectra >> 129 MB L2; no flush", "parallelism": "replicas"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "peak_source": peak_kind,
-                     "kernel": "ntt_pass_kernel (%d launches per multiply)" % pass_launches,
+                     "kernel": "transform passes (%d launches per multiply)" % pass_launches,
                      "algorithmic_bytes_per_launch": pass_bytes / max(1, pass_launches)},
         "issue_roofline": issue,
         "multiply_roofline": {"bytes_model": bm, "achieved_GBps": bm / (ms * 1e-3) / 1e9,
@@ -881,7 +883,7 @@ def run_radix3_leg(g, cudart, synth, lg, stream, logs):
     against n + 1 x n + 1 limbs (3 2^k + 1 coefficients), which take the
     power of two 2^(k+2): nearly the same product, a third more points."""
     out = {"sizes": [], "rule": "a product alone takes 3 2^k points from k = %s (GBNTT_RADIX3_MIN_LOG)"
-                                % os.environ.get("GBNTT_RADIX3_MIN_LOG", "20")}
+                                % os.environ.get("GBNTT_RADIX3_MIN_LOG", "17 on the 31-bit primes, 20")}
     flags = 0
     for k in logs:
         if k < 10 or (3 << k) + 1 > (1 << (lg + 1)):
@@ -928,7 +930,7 @@ def run_radix3_leg(g, cudart, synth, lg, stream, logs):
                              "radix3_launches": sum(by[x]["launches"] for x in by if x.startswith("radix3")),
                              "launch_breakdown": by,
                              "launch_breakdown_note": "one product with per-launch CUDA events (launches "
-                                                      "serialised, both primes on one stream)"})
+                                                      "serialised)"})
         for buf in (ra, rb, rc):
             buf.free()
     out["device_error_flags"] = flags
@@ -938,7 +940,7 @@ def run_radix3_leg(g, cudart, synth, lg, stream, logs):
 def run_negacyclic_leg(g, cudart, args, stream):
     """Negacyclic polynomial product mod X^N + 1 (the reference's crt_ntt
     negacyclic pipeline): N seeded 64-bit coefficients per operand, device
-    resident, three 64-bit primes, signed 256-bit outputs."""
+    resident, signed 256-bit outputs."""
     L = args.nega_log
     n = 1 << L
     df, dgb, do = cudart.DeviceBuffer(8 * n), cudart.DeviceBuffer(8 * n), cudart.DeviceBuffer(32 * n)
@@ -961,10 +963,10 @@ def run_negacyclic_leg(g, cudart, args, stream):
     ms = e0.elapsed_ms(e1) / steps
     for b in (df, dgb, do):
         b.free()
-    # bytes: coefficients in (16 N), three primes x (twist write, 2-pass
+    # bytes as over three 64-bit primes: coefficients in (16 N), three primes x (twist write, 2-pass
     # forward per operand, pointwise + inverse, finish read) and 32 N out
     bm = 16 * n + 3 * 8 * n * (2 + 2 * 2 * 2 + 3 + 2 + 1) + 32 * n
-    return {"ms": ms, "log_n": L, "coefficients": n, "primes": 3,
+    return {"ms": ms, "log_n": L, "coefficients": n,
             "bytes_model": bm, "bytes_model_GBps": bm / (ms * 1e-3) / 1e9,
             "output": "signed 256-bit coefficients (4 uint64 words each)",
             "api": "gbntt_negacyclic_mul_u64 (device pointers)"}
@@ -974,9 +976,9 @@ def _transfer_mode():
     if os.environ.get("GBNTT_ZERO_COPY", "1") == "0":
         return "cudaMemcpyAsync through the engine's staging buffer"
     if os.environ.get("GBNTT_STAGE_INPUTS", "1") == "0":
-        return ("zero copy: the first forward passes of both primes read the pinned operands and the carry "
+        return ("zero copy: the first forward passes read the pinned operands and the carry "
                 "kernel writes the pinned result over NVLink-C2C")
-    return ("operand A read over NVLink-C2C once by its first q0 pass (which leaves a copy in HBM for p3), "
+    return ("operand A read over NVLink-C2C once by its first stage, "
             "operand B pulled into HBM by a copy kernel on a second stream while A is transformed, product "
             "written to pinned memory by the carry kernel (zero copy)")
 

@@ -374,7 +374,8 @@ class Server:
 
 
 def set_prime_set(nprimes):
-    """2: q0 + the 32-bit p3 (default); 3: the reference's three 64-bit primes."""
+    """2: the fastest set for each length (default: 31-bit primes, q0 with p3
+    for the longest products); 3: the reference's three 64-bit primes."""
     _check(lib().gbntt_set_prime_set(int(nprimes)))
 
 

@@ -115,7 +115,9 @@ int gbntt_transform_log(size_t na, size_t nb);
 
 /* Pass plan for a transform of 2^log_n points: writes the pass sizes
  * (log2, outermost first) to passes[0..3] (room for GBNTT_MAX_PASSES ints)
- * and returns the pass count. */
+ * and returns the pass count. It is the plan of the 64-bit prime sets; the
+ * 31-bit set has defaults of its own, and an override (gbntt_set_plan) holds
+ * for all. */
 #define GBNTT_MAX_PASSES 4
 int gbntt_plan(int log_n, int *passes);
 
@@ -154,8 +156,9 @@ int gbntt_sqr_u32(uint32_t *d_c, const uint32_t *d_a, size_t na, void *stream);
  *   out[k] = sum_{i+j=k} f_i g_j - sum_{i+j=k+N} f_i g_j   (mod X^N + 1),
  * exact, as signed 256-bit two's complement integers (4 uint64 words per
  * coefficient, least significant first; |out[k]| < N 2^128). Device
- * pointers, stream-ordered; d_g == d_f squares. Three 64-bit primes
- * (modulus ~2^192). 5 <= log_n <= min(29, the initialised maximum). The
+ * pointers, stream-ordered; d_g == d_f squares. Three products of 32-bit
+ * halves on the 31-bit primes (log_n <= 24 and at most half the engine's
+ * length), else three 64-bit primes (modulus ~2^192). 5 <= log_n <= min(29, the initialised maximum). The
  * reference writes the unsigned residue modulo its four-prime modulus
  * (U256); here the value itself is written. */
 int gbntt_negacyclic_mul_u64(uint64_t *d_out, const uint64_t *d_f, const uint64_t *d_g, int log_n, void *stream);
@@ -194,8 +197,9 @@ int gbntt_server_stop(void);
 /* Packed mode: one 64-bit limb per coefficient (the reference engine's own
  * granularity, ntt/lib/arith/bigint.h:30-43). Operands and product are
  * 64-bit limb arrays (na, nb counted in 64-bit limbs; d_c gets na + nb
- * limbs); the transform length is the smallest power of two >= na + nb - 1,
- * half that of the 32-bit form for the same integers. Stream-ordered. */
+ * limbs). Products that the 31-bit primes take as 32-bit limbs run so; the
+ * others have one coefficient per limb over three 64-bit primes, the
+ * transform length the smallest power of two >= na + nb - 1. Stream-ordered. */
 int gbntt_mul_u64(uint64_t *d_c, const uint64_t *d_a, size_t na, const uint64_t *d_b, size_t nb, void *stream);
 int gbntt_sqr_u64(uint64_t *d_c, const uint64_t *d_a, size_t na, void *stream);
 int gbntt_mul_u64_host(uint64_t *c, const uint64_t *a, size_t na, const uint64_t *b, size_t nb);
@@ -223,7 +227,7 @@ int gbntt_device_errors(unsigned int *flags);
  * tests. d_out needs 3 * 2^log_n entries. */
 int gbntt_debug_forward(uint64_t *d_out, const uint32_t *d_in, size_t n, int log_n, void *stream);
 
-/* Residues of the 3 2^k-point transform path, two-prime set: mode 1, the
+/* Residues of the 3 2^k-point transform path of q0 with p3: mode 1, the
  * cyclic convolution of a and b of length 3 2^k (n_a + n_b - 1 <= 3 2^k)
  * before Garner; mode 0, 3 a after the forward and inverse radix-3 stages
  * alone (the 1/3 belongs to the inverse sub-transforms' scale). d_q0 receives 3 2^k q0 residues (uint64), d_p3 3 2^k p3
@@ -263,7 +267,9 @@ int gbntt_fill_operand(uint32_t *d, size_t n, uint64_t seed, void *stream);
  * 1 forward pass, 2 first inverse pass with the pointwise product,
  * 3 inverse pass, 4 Garner + carry, 5 the fused innermost passes: both
  * operands' last forward pass, the pointwise product and the first inverse
- * pass in one launch), its pass size log2 and its algorithmic
+ * pass in one launch, 6 and 7 the radix-3 stage forward and inverse, 8 whole
+ * products of up to 2^12 coefficients, 9 and 10 the outer stage forward and
+ * inverse), its pass size log2 and its algorithmic
  * bytes; gbntt_launch_log(0) stops and clears. gbntt_launch_records
  * synchronises and copies up to max_records entries; returns the count or
  * a negative GBNTT_* code. */
@@ -347,13 +353,15 @@ int gbntt_compute_e(long digits, char *out, size_t cap, double *phase_seconds);
 /* No counterpart in the reference (its engine always uses three 64-bit
  * primes). Primes used for products of 32-bit coefficients (gbntt_mul_u32,
  * batches, serving, the e pipeline and ntt_bigint_mul in its default
- * mode): 2 = q0 = 2^64 - 2^32 + 1 (64-bit residues) with p3 = 3 * 2^30 + 1
- * (32-bit residues), CRT modulus ~2^95.6 above every coefficient (< 2^93),
- * the default; 3 = the reference's three 64-bit primes. Products are
- * identical either way. Packed (64-bit coefficient) products always use
- * three 64-bit primes. The default comes from GBNTT_PRIMES (2 or 3) at
- * init. gbntt_prime_set returns 0 when no engine is initialised. Refused
- * (GBNTT_ERR_ARG) while the serving loop runs. */
+ * mode): 2 = the fastest set for the length, the default: three 31-bit
+ * primes (modulus ~2^92.6) for up to 2^29 coefficients with at most 2^28 limbs
+ * in the shorter operand, else q0 = 2^64 - 2^32 + 1 (64-bit residues) with
+ * p3 = 3 * 2^30 + 1 (32-bit residues), modulus ~2^95.6; 3 = the reference's
+ * three 64-bit primes (for packed and negacyclic products too). Products are
+ * identical either way. The default comes from GBNTT_PRIMES (2 or 3) at
+ * init; GBNTT_P31=0 leaves the 31-bit primes out. gbntt_prime_set returns 0
+ * when no engine is initialised. Refused (GBNTT_ERR_ARG) while the serving
+ * loop runs. */
 int gbntt_set_prime_set(int nprimes);
 int gbntt_prime_set(void);
 
