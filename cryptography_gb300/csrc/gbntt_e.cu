@@ -356,7 +356,8 @@ constexpr size_t kRecipHostLimbs = 64;
 // piece x gives its two level-(j-1) pieces q = floor(x / d_j) (the leading
 // digits) and r = x - q d_j. One CTA takes one piece of level `top` and
 // splits it level by level down to `low`, all in shared memory, then prints
-// the pieces of level low - 1 (9 2^low digits each, one thread per piece).
+// the pieces of level low - 1 (9 2^low digits each, one thread per piece), or
+// splits one level and leaves the two pieces in global memory.
 //
 // A split is Barrett's reduction with mu_j = floor(beta^(2n) / d_j) (n + 1
 // limbs, beta = 2^32; HAC algorithm 14.42): q^ = floor(floor(x / beta^(n-1))
@@ -379,6 +380,12 @@ constexpr size_t kRecipHostLimbs = 64;
 // 256, 6.2 with 512; 523 pieces 13.4, 13.5 and 14.
 constexpr int kDecWide = 512;        // at most one CTA per SM
 constexpr int kDecThreads = 256;
+// Levels from kDecSplitMin on are split by a launch each while their pieces
+// leave half of the SMs idle: each piece then has an SM to itself one level
+// earlier (to_decimal of 3000 limbs 0.70 -> 0.65 ms, of 250007 3.78 -> 3.69).
+// Below, a level costs no more than the launch (300 limbs, levels from 8 on:
+// 0.345 -> 0.353).
+constexpr int kDecSplitMin = 10;
 constexpr int kDecCols = 5;          // product columns per thread item; odd, so that the
                                      // lanes' operand reads (stride kDecCols) hit distinct banks
 constexpr int kDecPad = kDecCols;    // zero limbs on either side of d_j and mu_j in the table
@@ -395,8 +402,10 @@ struct DecLevel {
 };
 
 struct DecArgs {
-    const uint32_t *pieces;   // pieces of level `top`, stride lv[top].stride
+    const uint32_t *pieces;   // piece base of level `top` and on, stride lv[top].stride
+    long long base;
     long long first;          // CTA b converts piece first + b
+    uint32_t *split;          // if set: level `top` (= low) alone, CTA b's two pieces to split + 2 b lv[top - 1].stride
     int top, low;
     int leaf_stride;          // stride of a level low - 1 piece
     int buf_limbs;            // limbs of each of the two piece buffers
@@ -563,7 +572,7 @@ __global__ void __launch_bounds__(THREADS) dec_block_kernel(const DecArgs A)
     const long long piece = A.first + blockIdx.x;
     {
         const int S = A.lv[A.top].stride;
-        const uint32_t *src = A.pieces + piece * S;
+        const uint32_t *src = A.pieces + (piece - A.base) * S;
         for (int i = tid; i < S; i += THREADS) cur[i] = src[i];
     }
     __syncthreads();
@@ -626,6 +635,12 @@ __global__ void __launch_bounds__(THREADS) dec_block_kernel(const DecArgs A)
         uint32_t *sw = cur;
         cur = nxt;
         nxt = sw;
+    }
+    if (A.split) {
+        const int n = 2 * A.lv[A.top - 1].stride;
+        uint32_t *dst = A.split + (long long)blockIdx.x * n;
+        for (int i = tid; i < n; i += THREADS) dst[i] = cur[i];
+        return;
     }
     // print the level low - 1 pieces: 9 2^low digits each, by repeated
     // division by 10^9 in place
@@ -1726,7 +1741,6 @@ struct Pipe {
         const long long TD = 9LL << (J + 1);      // padded digit count
         const long long Z = TD - dub;             // leading digits known to be zero
         const int top = std::min(J, dec_top_level());
-        const int low = std::max(0, top - (kDecLeafLog - 1));
         const DecConst &K = dec_constants();
         DTab<char> dig((size_t)TD);
         // d_j = 10^(9 2^j), nd_j limbs; pieces of level j are below d_j^2 and
@@ -1786,43 +1800,58 @@ struct Pipe {
             Stopwatch sw;
             DBuf ct(K.tab.size());
             ECK(cudaMemcpyAsync(ct.p, K.tab.data(), K.tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, g_st));
+            int dev = 0, sms = 0, cap = 0;
+            ECK(cudaGetDevice(&dev));
+            ECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            ECK(cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
             DecArgs a{};
-            a.pieces = lev.p;
-            a.first = Z / (9LL << (top + 1));
-            a.top = top;
-            a.low = low;
-            a.leaf_stride = low > 0 ? K.lv[low - 1].stride : 2;
             a.ctab = ct.p;
             for (int j = 0; j <= kDecMaxTop; j++) a.lv[j] = K.lv[j];
             a.digits = dig.p;
             a.err = d_err;
-            long long buf = 0, blk = 0;
-            for (int j = low - 1; j <= top; j++)
-                buf = std::max(buf, (1LL << (top - j)) * (j >= 0 ? K.lv[j].stride : 2));
-            for (int j = low; j <= top; j++) blk = std::max(blk, (1LL << (top - j)) * K.lv[j].nblk);
-            a.buf_limbs = (int)buf;
-            a.blk_items = (int)blk;
-            const size_t smem = (size_t)(2 * buf + blk * (kDecCols + 2)) * sizeof(uint32_t);
-            const long long ncta = (1LL << (J - top)) - a.first;
-            int dev = 0, sms = 0;
-            ECK(cudaGetDevice(&dev));
-            ECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            const bool wide = ncta <= sms;
-            const int threads = wide ? kDecWide : kDecThreads;
-            void (*const kernel)(const DecArgs) = wide ? dec_block_kernel<kDecWide> : dec_block_kernel<kDecThreads>;
-            if (smem > 48 * 1024) {
-                int cap = 0;
-                ECK(cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+            // Pieces of level t below which the first Z digits lie, split down to level low.
+            size_t smem = 0;
+            auto launch = [&](int t, int low, uint32_t *split) {
+                a.pieces = lev.p;
+                a.first = Z / (9LL << (t + 1));
+                a.top = t;
+                a.low = low;
+                a.split = split;
+                a.leaf_stride = low > 0 ? K.lv[low - 1].stride : 2;
+                long long buf = 0, blk = 0;
+                for (int j = low - 1; j <= t; j++)
+                    buf = std::max(buf, (1LL << (t - j)) * (j >= 0 ? K.lv[j].stride : 2));
+                for (int j = low; j <= t; j++) blk = std::max(blk, (1LL << (t - j)) * K.lv[j].nblk);
+                a.buf_limbs = (int)buf;
+                a.blk_items = (int)blk;
+                smem = (size_t)(2 * buf + blk * (kDecCols + 2)) * sizeof(uint32_t);
+                const long long ncta = (1LL << (J - t)) - a.first;
+                const bool wide = ncta <= sms;
+                const int threads = wide ? kDecWide : kDecThreads;
+                void (*const kernel)(const DecArgs) = wide ? dec_block_kernel<kDecWide> : dec_block_kernel<kDecThreads>;
                 if (smem > (size_t)cap) efail(GBNTT_ERR_SIZE, "decimal block of level %d needs %zu bytes of shared "
-                                              "memory (%d available)", top, smem, cap);
-                ECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                              "memory (%d available)", t, smem, cap);
+                if (smem > 48 * 1024)
+                    ECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                kernel<<<(unsigned)ncta, (unsigned)threads, smem, g_st>>>(a);
+                ECK(cudaGetLastError());
+                return ncta;
+            };
+            int t = top;
+            for (; t >= kDecSplitMin; t--) {
+                const long long first = Z / (9LL << (t + 1)), ncta = (1LL << (J - t)) - first;
+                if (2 * ncta > sms) break;
+                DBuf child((size_t)(2 * ncta) * K.lv[t - 1].stride);
+                launch(t, t, child.p);
+                lev = std::move(child);
+                a.base = 2 * first;
             }
-            kernel<<<(unsigned)ncta, (unsigned)threads, smem, g_st>>>(a);
-            ECK(cudaGetLastError());
+            const int low = std::max(0, t - (kDecLeafLog - 1));
+            const long long ncta = launch(t, low, nullptr);
             if (prof) {
                 sync();
-                fprintf(stderr, "to_decimal levels %d..%d in one kernel: %lld pieces, %zu bytes shared, %.2f ms\n",
-                        top, low, ncta, smem, sw.lap() * 1e3);
+                fprintf(stderr, "to_decimal levels %d..%d, %d on in one kernel: %lld pieces, %zu bytes shared, %.2f ms\n",
+                        top, low, t, ncta, smem, sw.lap() * 1e3);
             }
         }
         // Z under-counts the leading zeros by at most two (the digit bound

@@ -1,5 +1,6 @@
-"""Decimal conversions on both sides of the line between one in-memory piece
-per multiprocessor and more, digit for digit: D random digits, D a multiple of
+"""Decimal conversions on both sides of the lines between one in-memory piece
+per multiprocessor and more, and between pieces split by launches of their own
+and in one, digit for digit: D random digits, D a multiple of
 a block's digits and one off, and all nines."""
 import random
 import sys
@@ -12,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("top,pieces", [(0, 1), (0, 152), (0, 153), (3, 151), (3, 152), (3, 153), (3, 400), (7, 40),
-                                        (7, 170), (11, 1), (11, 2)])
+                                        (7, 170), (11, 1), (11, 2), (8, 20), (8, 75), (8, 76), (8, 77), (9, 37), (9, 39), (10, 5), (11, 5), (12, 1)])
 def test_pieces_per_multiprocessor(engine, top, pieces, monkeypatch):
     monkeypatch.setenv("GBNTT_DEC_TOP", str(top))
     if hasattr(sys, "set_int_max_str_digits"):
