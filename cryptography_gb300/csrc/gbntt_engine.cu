@@ -289,17 +289,21 @@ static void free_pass_tables()
     g_ptw_bytes = 0;
 }
 
-// Per-length plan overrides (set by gbntt_set_plan, e.g. from an autotuner):
-// [log_n][0] = pass count (0: default plan), [1..kMaxPasses] = pass sizes.
+// Per-length plan overrides: [log_n][0] = pass count (0: default plan),
+// [1..kMaxPasses] = pass sizes. The 31-bit primes have a table of their own:
+// gbntt_set_plan writes both, the autotuner the one whose passes it timed.
 static int g_plan_override[kMaxLog + 1][1 + kMaxPasses];
+static int g_plan31_override[kMaxLog + 1][1 + kMaxPasses];
+
+static int read_override(const int *o, int *p)
+{
+    for (int i = 0; i < o[0]; i++) p[i] = o[1 + i];
+    return o[0];
+}
 
 int plan_passes(int log_n, int *p)
 {
-    if (log_n >= 0 && log_n <= kMaxLog && g_plan_override[log_n][0] > 0) {
-        const int np = g_plan_override[log_n][0];
-        for (int i = 0; i < np; i++) p[i] = g_plan_override[log_n][1 + i];
-        return np;
-    }
+    if (log_n >= 0 && log_n <= kMaxLog && g_plan_override[log_n][0] > 0) return read_override(g_plan_override[log_n], p);
     if (log_n <= kMaxPassLog) { p[0] = log_n; return 1; }
     // 2^14 .. 2^30: the plans gbntt_autotune measured fastest on GB300 for
     // 2^(L-1) x 2^(L-1)-limb products (two-prime set, innermost passes
@@ -326,8 +330,8 @@ int plan_passes(int log_n, int *p)
     return 2;
 }
 
-// Pass plan of a 2^log_n-point transform of the 31-bit prime set: the
-// override, or the fastest of the plans gbntt_autotune times.
+// Pass plan of a 2^log_n-point transform of the 31-bit prime set (log_n <=
+// kP31MaxLog): the override, or the fastest of the plans gbntt_autotune times.
 static int p31_plan(int log_n, int *p)
 {
     constexpr int kLo = 11;
@@ -337,7 +341,11 @@ static int p31_plan(int log_n, int *p)
         {3, 5, 6, 8}, {3, 5, 7, 8}, {3, 7, 7, 7}, {3, 7, 7, 8},  // 2^19 .. 2^22
         {3, 8, 7, 8}, {3, 8, 8, 8}, {3, 9, 8, 8},                // 2^23 .. 2^25
     };
-    if (log_n < kLo || g_plan_override[log_n][0] > 0) return plan_passes(log_n, p);
+    if (g_plan31_override[log_n][0] > 0) return read_override(g_plan31_override[log_n], p);
+    if (log_n < kLo) {   // (one pass: every length here is a pass size)
+        p[0] = log_n;
+        return 1;
+    }
     const signed char *t = kTuned[log_n - kLo];
     for (int i = 0; i < t[0]; i++) p[i] = t[1 + i];
     return t[0];
@@ -2743,6 +2751,8 @@ int gbntt_transform_log(size_t na, size_t nb) { return (na == 0 || nb == 0) ? 0 
 int gbntt_plan(int log_n, int *passes)
 {
     if (log_n < kMinLog || log_n > kMaxLog || !passes) return 0;
+    if (use_p31(log_n) && !use_block(log_n) && g_plan31_override[log_n][0] > 0)
+        return read_override(g_plan31_override[log_n], passes);
     return plan_passes(log_n, passes);
 }
 const char *gbntt_last_error(void) { return g_err; }
@@ -2751,7 +2761,11 @@ int gbntt_set_plan(int log_n, int npasses, const int *passes)
 {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     if (log_n < kMinLog || log_n > kMaxLog) { set_err("gbntt_set_plan: log_n %d out of range", log_n); return GBNTT_ERR_ARG; }
-    if (npasses == 0) { g_plan_override[log_n][0] = 0; invalidate_wave_graphs(); return GBNTT_OK; }
+    if (npasses == 0) {
+        g_plan_override[log_n][0] = g_plan31_override[log_n][0] = 0;
+        invalidate_wave_graphs();
+        return GBNTT_OK;
+    }
     if (npasses < 1 || npasses > kMaxPasses || !passes) {
         set_err("gbntt_set_plan: 1 to %d passes", kMaxPasses);
         return GBNTT_ERR_ARG;
@@ -2765,8 +2779,10 @@ int gbntt_set_plan(int log_n, int npasses, const int *passes)
         sum += passes[i];
     }
     if (sum != log_n) { set_err("gbntt_set_plan: pass sizes sum to %d, not %d", sum, log_n); return GBNTT_ERR_ARG; }
-    g_plan_override[log_n][0] = npasses;
-    for (int i = 0; i < npasses; i++) g_plan_override[log_n][1 + i] = passes[i];
+    for (auto *o : {g_plan_override[log_n], g_plan31_override[log_n]}) {
+        o[0] = npasses;
+        for (int i = 0; i < npasses; i++) o[1 + i] = passes[i];
+    }
     invalidate_wave_graphs();
     return GBNTT_OK;
 }
@@ -2775,7 +2791,9 @@ int gbntt_set_plan(int log_n, int npasses, const int *passes)
 // pass plan of 1 to kMaxPasses passes (each 2^5 .. 2^10 points) on a
 // synthetic 2^(L-1) x 2^(L-1)-limb product through the normal multiply path
 // (CUDA events on the engine stream, best of `reps` after a warm-up), and
-// install the fastest through the plan-override table.
+// install the fastest through the plan-override table of the primes that the
+// product ran on. A product that runs no passes of 2^L points (whole in one
+// CTA, or through the outer stage) is timed once, and no plan is installed.
 // plans[(1 + kMaxPasses) i ...] receives (pass count, sizes...) and ms[i]
 // its time for L = log_lo + i.
 int gbntt_autotune(int log_lo, int log_hi, int reps, int *plans, float *ms)
@@ -2796,10 +2814,15 @@ int gbntt_autotune(int log_lo, int log_hi, int reps, int *plans, float *ms)
         uint32_t *da = g.d_io, *db = da + half, *dc = db + half;
         CK(launch_fill_splitmix(da, (long long)half, 0x5eed0000u + L, g.stream));
         CK(launch_fill_splitmix(db, (long long)half, 0x5eed1000u + L, g.stream));
+        int *const target = use_p31(L) ? g_plan31_override[L] : g_plan_override[L];
+        const bool planless = use_block(L) || p31_outer_blocks(half, half) > 0;
         // every composition of L into 1..kMaxPasses parts of 5..10
         typedef std::array<int, 1 + kMaxPasses> Plan;
         std::vector<Plan> cands;
         Plan cur{};
+        auto install = [&](const Plan &c) {
+            if (!planless) std::copy(c.begin(), c.end(), target);
+        };
         auto extend = [&](auto &&self, int depth, int left) -> void {
             if (left == 0 && depth > 0) {
                 Plan c{};
@@ -2814,12 +2837,16 @@ int gbntt_autotune(int log_lo, int log_hi, int reps, int *plans, float *ms)
                 self(self, depth + 1, left - p);
             }
         };
-        extend(extend, 0, L);
+        if (planless) {
+            cur[0] = plan_passes(L, &cur[1]);
+            cands.push_back(cur);
+        } else {
+            extend(extend, 0, L);
+        }
         float best = 1e30f;
         Plan best_plan{};
         for (const auto &c : cands) {
-            g_plan_override[L][0] = c[0];
-            for (int i = 0; i < kMaxPasses; i++) g_plan_override[L][1 + i] = c[1 + i];
+            install(c);
             if ((rc = mul_dev(dc, da, half, db, half, g.stream)) != GBNTT_OK) break;   // warm-up
             float t_min = 1e30f;
             for (int r = 0; r < reps && rc == GBNTT_OK; r++) {
@@ -2839,8 +2866,7 @@ int gbntt_autotune(int log_lo, int log_hi, int reps, int *plans, float *ms)
             CK(cudaDeviceSynchronize());
             free_pass_tables();
         }
-        g_plan_override[L][0] = best_plan[0];
-        for (int i = 0; i < kMaxPasses; i++) g_plan_override[L][1 + i] = best_plan[1 + i];
+        install(best_plan);
         if (plans)
             for (int i = 0; i <= kMaxPasses; i++) plans[(1 + kMaxPasses) * (L - log_lo) + i] = best_plan[i];
         if (ms) ms[L - log_lo] = best;

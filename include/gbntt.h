@@ -115,22 +115,29 @@ int gbntt_transform_log(size_t na, size_t nb);
 
 /* Pass plan for a transform of 2^log_n points: writes the pass sizes
  * (log2, outermost first) to passes[0..3] (room for GBNTT_MAX_PASSES ints)
- * and returns the pass count. It is the plan of the 64-bit prime sets; the
- * 31-bit set has defaults of its own, and an override (gbntt_set_plan) holds
- * for all. */
+ * and returns the pass count. By default it is the plan of the 64-bit prime
+ * sets (the 31-bit set has defaults of its own); an override that products of
+ * that length run by is reported instead. */
 #define GBNTT_MAX_PASSES 4
 int gbntt_plan(int log_n, int *passes);
 
 /* Override the pass plan of transforms of 2^log_n points (1 to 4 passes,
  * each of 2^5 .. 2^10 points, sizes summing to log_n, outermost first);
- * npasses = 0 restores the default plan. Used by the autotuner. */
+ * npasses = 0 restores the default plan. The override holds for every prime
+ * set; a product that runs no passes of that length (gbntt_autotune) does not
+ * see it. */
 int gbntt_set_plan(int log_n, int npasses, const int *passes);
 
 /* Autotuner (the reference picks its transform factorisation by hand): for
  * each transform length 2^L, log_lo <= L <= log_hi <= the initialised
  * maximum, times every pass plan of 1 to 4 passes of 2^5 .. 2^10 points on a
  * synthetic product (best of `reps` runs after a warm-up, CUDA events) and
- * installs the fastest as that length's plan (as gbntt_set_plan does).
+ * installs the fastest as that length's plan for the primes the product ran
+ * on: with the default set the 31-bit ones where 13 <= L <= 25, else q0 with
+ * p3; with prime set 3 the 64-bit ones. On the 31-bit primes products of up
+ * to 2^12 coefficients run whole in one kernel and those above 2^25 as
+ * transforms of 2^25 points, without passes of 2^L points: such a length is
+ * timed as it is, keeps its plan, and that plan is what plans receives.
  * plans (may be NULL) receives 1 + GBNTT_MAX_PASSES ints per length: pass
  * count, then the sizes (unused entries 0);
  * ms (may be NULL) the winning time in milliseconds. Synchronous. */
