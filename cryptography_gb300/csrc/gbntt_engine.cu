@@ -1902,6 +1902,7 @@ static int batch_mul(uint32_t *const *d_c, const uint32_t *const *d_a, const siz
     };
     std::vector<Keyed> all;
     std::vector<Split> splits;
+    std::vector<int> alone;   // products that run by themselves, after the waves
     size_t split_words = 0;
     uint32_t *split_buf = nullptr;
     all.reserve(count);
@@ -1958,7 +1959,7 @@ static int batch_mul(uint32_t *const *d_c, const uint32_t *const *d_a, const siz
             // longer than a 31-bit transform: it fills the GPU by itself, and
             // a wave of such products would run on q0 with p3 (a pair sharing
             // its right operand 86 ms at 2^28 limbs, two products alone 68)
-            rc = mul_dev(d_c[i], d_a[i], na[i], d_b[i], nb[i], st);
+            alone.push_back(i);   // (once every product of the batch is known to fit)
             continue;
         }
         all.push_back({L, (long long)i, {d_c[i], d_a[i], d_b[i], na[i], nb[i]}});
@@ -2053,6 +2054,10 @@ static int batch_mul(uint32_t *const *d_c, const uint32_t *const *d_a, const siz
                 rc = batch_wave(x, items.data(), W, L, st, g.stream2, r3 != 0);
             }
             pos = end;
+        }
+        for (size_t k = 0; k < alone.size() && rc == GBNTT_OK; k++) {
+            const int i = alone[k];
+            rc = mul_dev(d_c[i], d_a[i], na[i], d_b[i], nb[i], st);
         }
     }
     if (split_buf) {
