@@ -326,13 +326,15 @@ def negacyclic_mul(f, g):
 
 def _c_array(ctype, code, n, values):
     # n integers as a C array; array.array converts a list about four times
-    # faster than the ctypes constructor, which takes what it refuses
-    try:
-        a = array.array(code, values)
-        if len(a) == n:
-            return (ctype * n).from_buffer(a)
-    except (OverflowError, TypeError):
-        pass
+    # faster than the ctypes constructor, which takes what it refuses (any other
+    # iterable too: it may be consumed, or be bytes, which array takes as words)
+    if isinstance(values, (list, tuple, np.ndarray)):
+        try:
+            a = array.array(code, values)
+            if len(a) == n:
+                return (ctype * n).from_buffer(a)
+        except (OverflowError, TypeError):
+            pass
     return (ctype * n)(*values)
 
 
