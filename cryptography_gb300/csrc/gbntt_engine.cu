@@ -767,10 +767,13 @@ static bool use_p31(int L) { return g.p31 && g.prime_set == 2 && L <= kP31MaxLog
 // Number of 2^25-point transforms of a product of more than 2^25
 // coefficients on the 31-bit prime set (gbntt_p31_outer.cu), 0 if it does not
 // take it: up to 2^29 coefficients and 2^28 limbs in the shorter operand,
-// whose coefficients are below 2^92.
+// whose coefficients are below 2^92. Never 3: 3 2^25 points are the radix-3
+// stage's, and where that is switched off such a product takes four blocks.
 static int p31_outer_blocks(size_t na, size_t nb)
 {
-    const size_t need = na + nb - 1, blocks = (need + ((size_t)1 << kP31MaxLog) - 1) >> kP31MaxLog;
+    const size_t need = na + nb - 1;
+    size_t blocks = (need + ((size_t)1 << kP31MaxLog) - 1) >> kP31MaxLog;
+    if (blocks == 3) blocks = 4;
     const bool fits = blocks > 1 && blocks <= (size_t)kP31MaxOuter &&
                       std::min(na, nb) <= (size_t)1 << 28 && (blocks << kP31MaxLog) <= g.n_max;
     return g.p31 && g.prime_set == 2 && fits ? (int)blocks : 0;
@@ -1195,8 +1198,8 @@ static int copy_operand(const StageJob &j)
 }
 
 // Residues of W products a b in A's spectra, ready for the carry kernel:
-// transforms of R 2^L points, R = 1, 3 (the radix-3 stage) or, with W = 1
-// and L = 25, up to kP31MaxOuter (the outer stage). copy_b (optional): B's
+// transforms of R 2^L points, R = 1, 3 (always the radix-3 stage) or, with
+// W = 1 and L = 25, p31_outer_blocks' (the outer stage). copy_b (optional): B's
 // limbs are copied on the copy stream once A's outer stage, if it has one, has
 // read A, which may be in host memory; A is transformed meanwhile.
 static int p31_products(const P31Op &A, const P31Op &B, size_t stride, int L, int R, P31Right right, unsigned *ctl,
@@ -1440,7 +1443,7 @@ static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint
                        cudaStream_t st, const StageJob *stage_b, uint32_t *stage_a)
 {
     const bool square = (d_a == d_b && na == nb);
-    const bool outer = L == kP31MaxLog && R > 1 && R != 3;   // (R = 3 is the radix-3 stage)
+    const bool outer = R > 1 && R != 3;   // (R = 3 is the radix-3 stage)
     if (stage_a && !outer) {
         CK(launch_copy_words(stage_a, d_a, (long long)na, g.sms * 4, st));
         d_a = stage_a;

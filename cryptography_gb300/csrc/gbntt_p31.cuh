@@ -335,8 +335,8 @@ struct P31R3Args {
 };
 cudaError_t launch_p31_radix3(bool inverse, const P31R3Args &a, cudaStream_t st);
 
-// Outer stage of a product of up to R 2^25 coefficients: spectrum m at
-// spec[prime] + m 2^25.
+// Outer stage of a product of up to R 2^25 coefficients (R = 2, 4 .. 16):
+// spectrum m at spec[prime] + m 2^25.
 constexpr int kP31MaxOuter = 16;
 struct P31OuterArgs {
     uint32_t *spec[3];

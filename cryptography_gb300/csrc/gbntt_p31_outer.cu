@@ -2,10 +2,11 @@
 // primes.
 //
 // The primes' roots of unity end at 2^25, so a product of up to R M
-// coefficients (M = 2^25, 2 <= R <= 16) is computed modulo R polynomials
-// X^M - c_m that do have M-th roots of c_m: c_m = gamma^m, gamma = g^M, for a
-// g of order d M with d = (p - 1) / M = 60, 54 and 63 in the three primes
-// (gamma has order d >= R, so the c_m differ).
+// coefficients (M = 2^25; R = 2, 4 .. 16, 3 M points being the radix-3
+// stage's) is computed modulo R polynomials X^M - c_m that do have M-th roots
+// of c_m: c_m = gamma^m, gamma = g^M, for a g of order d M with d = (p - 1) / M
+// = 60, 54 and 63 in the three primes (gamma has order d >= R, so the c_m
+// differ).
 //   forward  y_m[j] = g^(jm) sum_r x[j + r M] gamma^(rm)     (A mod X^M - c_m
 //            under X -> g^m X, a cyclic convolution of length M)
 //   inverse  t_m = z_m[j] g^(-jm), x[j + r M] = sum_m V^-1[r][m] t_m with the
@@ -233,7 +234,6 @@ cudaError_t launch_p31_outer(int R, bool inverse, const P31OuterArgs &a, cudaStr
 {
     switch (R) {
     case 2: return launch_r<2>(inverse, a, st);
-    case 3: return launch_r<3>(inverse, a, st);
     case 4: return launch_r<4>(inverse, a, st);
     case 5: return launch_r<5>(inverse, a, st);
     case 6: return launch_r<6>(inverse, a, st);
@@ -279,7 +279,7 @@ cudaError_t p31_outer_init()
 {
     std::vector<uint32_t> h((size_t)(kMaxR + 1) * 3 * kMaxR * kMaxR, 0);
     for (int R = 2; R <= kMaxR; R++)
-        for (int k = 0; k < 3; k++) {
+        for (int k = 0; k < 3 && R != 3; k++) {
             const uint64_t p = kP31[k], gamma = p31_pow(outer_g(k), kM, p);
             uint32_t *dst = h.data() + ((size_t)R * 3 + k) * kMaxR * kMaxR;
             auto mont = [&](uint64_t x) { return (uint32_t)((x << 32) % p); };
