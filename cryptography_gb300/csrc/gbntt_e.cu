@@ -382,7 +382,7 @@ constexpr int kDecWide = 512;        // at most one CTA per SM
 constexpr int kDecThreads = 256;
 // Levels from kDecSplitMin on are split by a launch each while their pieces
 // leave half of the SMs idle: each piece then has an SM to itself one level
-// earlier (to_decimal of 3000 limbs 0.70 -> 0.65 ms, of 250007 3.78 -> 3.69).
+// earlier (to_decimal of 3000 limbs 0.70 -> 0.65 ms, of 250007 3.76 -> 3.72).
 // Below, a level costs no more than the launch (300 limbs, levels from 8 on:
 // 0.345 -> 0.353).
 constexpr int kDecSplitMin = 10;
@@ -1524,7 +1524,7 @@ struct Pipe {
     // at most two below beta^(2n') / (d^2 2^s'), the dropped part is below
     // 2 beta^(n+1) / beta^(2n-2) < 1 (n' >= 2n - 1, n >= 4): Y is exact or
     // one below, which leaves the quotient estimate of divide() at most two
-    // below the quotient, within its two correction rounds.
+    // below the quotient, within the three multiples it takes off.
     void derive_divisor(Divisor &D, const uint32_t *d, size_t nd, const Divisor &up)
     {
         if (nd < 4 || up.k != up.nd || up.nd + 1 < 2 * nd) efail(GBNTT_ERR_ARG, "divisor derivation out of range");

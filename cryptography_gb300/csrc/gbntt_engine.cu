@@ -65,9 +65,10 @@ struct PrimeSet {
 static const PrimeSet kSet2 = {2, {4, 3, 0}};       // lazy normal-form q0 + p3
 static const PrimeSet kSet2m = {2, {0, 3, 0}};      // Montgomery q0 + p3
 static const PrimeSet kSet3 = {3, {0, 1, 2}};
-// The 31-bit primes (indices 5..7, gbntt_p31.cuh): every product of 32-bit
-// coefficients of up to 3 2^25 points, unless three 64-bit primes or lazy q0
-// are asked for. All three share their launches.
+// The 31-bit primes (indices 5..7, gbntt_p31.cuh): products of 32-bit
+// coefficients of up to 3 2^25 points, and through the outer stage up to 2^29
+// coefficients, unless three 64-bit primes or lazy q0 are asked for (served
+// and cyclic products: up to 3 2^25 points). All three share their launches.
 static const PrimeSet kSet31 = {3, {5, 6, 7}};
 
 struct Engine {
@@ -1179,8 +1180,11 @@ static int p31_outer(const P31Op &op, size_t stride, int R, bool inverse, cudaSt
     return GBNTT_OK;
 }
 
-// Host -> device copy of the second operand, issued once the first operand's
-// first pass or outer stage has read its limbs (both share the host link).
+// Host -> device copy of the second operand. On the 31-bit primes it runs
+// before both transforms, or beside the first one's on the copy stream (from
+// kCopyBeside points on), there after the first operand's outer or radix-3
+// stage; on q0 with p3 beside the first one's, after its first pass (both
+// operands share the host link).
 struct StageJob {
     uint32_t *dst = nullptr;
     const uint32_t *src = nullptr;   // device-mapped pinned memory, or a host pointer
@@ -1473,9 +1477,9 @@ static int mul_dev_p31(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint
     return carry(kSet31, d_c, na + nb, g.d_spec, g.n_max, L, st, (long long)R << L, (long long)std::min(na, nb));
 }
 
-// stage_a (optional): HBM copy of A made by its first pass (see forward).
-// stage_b (optional): copy of B into d_b, run on the copy stream while A is
-// transformed.
+// stage_a (optional): where an A in host memory goes, unless the outer stage
+// reads it in place (mul_dev_p31; q0 with p3: its first pass copies it, see
+// forward). stage_b (optional): copy of B into d_b.
 static int mul_dev(uint32_t *d_c, const uint32_t *d_a, size_t na, const uint32_t *d_b, size_t nb, cudaStream_t st,
                    const StageJob *stage_b = nullptr, uint32_t *stage_a = nullptr)
 {
@@ -2351,17 +2355,12 @@ static int read_errors(unsigned *flags)
     return GBNTT_OK;
 }
 
-// Host-pointer product through the staging buffer (a, b, c contiguous).
-// Device address of page-locked host memory (NVLink-C2C makes it directly
-// readable and writable by kernels), or nullptr for other memory.
 // Negacyclic product modulo X^N + 1 (N = 2^L) of two N-coefficient
-// polynomials with 64-bit coefficients, over the three 64-bit primes:
-// twist, the cyclic pass chain, the fused pointwise product and inverse,
-// then untwist + Garner to signed 256-bit coefficients (reference
-// pipeline_negacyclic, ntt/lib/main.hip:557-684).
+// polynomials with 64-bit coefficients on the 31-bit primes: three products
+// of 32-bit halves (gbntt_p31_nega.cu) from twist to signed 256-bit
+// coefficients.
 static int negacyclic_p31(uint64_t *d_out, const uint64_t *d_f, const uint64_t *d_g, int L, cudaStream_t st)
 {
-    // three products of 2^L points side by side (gbntt_p31_nega.cu)
     const bool square = d_f == d_g;
     const size_t N = (size_t)1 << L, stride = 3 * N / 2;   // 3 N 32-bit words per prime
     uint64_t *specA = g.d_spec, *specB = g.d_spec + 3 * stride;
@@ -2393,6 +2392,10 @@ static int negacyclic_p31(uint64_t *d_out, const uint64_t *d_f, const uint64_t *
     return GBNTT_OK;
 }
 
+// The same by the 31-bit primes, or where they don't take it over the three
+// 64-bit primes: twist, the cyclic pass chain, the fused pointwise product and
+// inverse, then untwist + Garner to signed 256-bit coefficients (reference
+// pipeline_negacyclic, ntt/lib/main.hip:557-684).
 static int negacyclic_dev(uint64_t *d_out, const uint64_t *d_f, const uint64_t *d_g, int L, cudaStream_t st)
 {
     if (!g.ready) { set_err("engine not initialised"); return GBNTT_ERR_NOT_INIT; }
@@ -2452,6 +2455,8 @@ static int negacyclic_dev(uint64_t *d_out, const uint64_t *d_f, const uint64_t *
     return GBNTT_OK;
 }
 
+// Device address of page-locked host memory (NVLink-C2C makes it directly
+// readable and writable by kernels), or nullptr for other memory.
 static void *pinned_device_ptr(const void *p)
 {
     cudaPointerAttributes at;
@@ -2516,6 +2521,7 @@ static int mul_host_short(uint32_t *c, const uint32_t *a, size_t na, const uint3
     return device_failure(h[0]);
 }
 
+// Host-pointer product through the staging buffer (a, b, c contiguous).
 static int mul_host(uint32_t *c, const uint32_t *a, size_t na, const uint32_t *b, size_t nb,
                     const uint32_t *dev_a, const uint32_t *dev_b)
 {
@@ -2534,12 +2540,11 @@ static int mul_host(uint32_t *c, const uint32_t *a, size_t na, const uint32_t *b
     const uint32_t *ua = dev_a, *ub = dev_b;
     // Zero copy: a pinned result is written by the carry kernel over
     // NVLink-C2C. Pinned operands: without stage_inputs the first forward
-    // passes read them in place, each limb once per prime (the outer stage:
-    // once). With it (default) each limb crosses the link once: A is read in
-    // place by the outer stage, or copied first, or (q0 with p3) copied by its
-    // first q0 pass for p3's, and B is pulled into HBM by a copy kernel, for
-    // long products on the copy stream while A is being transformed. Pageable
-    // operands go through cudaMemcpyAsync.
+    // passes read them in place, each limb once per prime (the outer and the
+    // radix-3 stage: once). With it (default) each limb crosses the link once:
+    // A is copied first, or read in place by the outer stage, or (q0 with p3)
+    // copied by its first q0 pass for p3's; when B is copied stands at
+    // StageJob. Pageable operands go through cudaMemcpyAsync.
     if (!ua && g.zero_copy && !g.stage_inputs) ua = (const uint32_t *)pinned_device_ptr(a);
     if (!ub && !square && g.zero_copy && !g.stage_inputs) ub = (const uint32_t *)pinned_device_ptr(b);
     uint32_t *uc = g.zero_copy ? (uint32_t *)pinned_device_ptr(c) : nullptr;
@@ -2552,7 +2557,7 @@ static int mul_host(uint32_t *c, const uint32_t *a, size_t na, const uint32_t *b
     int rs;
     uint32_t *stage_a = nullptr;
     if (!ua && g.zero_copy && g.stage_inputs && (ua = (const uint32_t *)pinned_device_ptr(a)) != nullptr) {
-        stage_a = da;   // A's first pass reads it over C2C once and leaves a copy in HBM for the other prime
+        stage_a = da;
     } else if (!ua) {
         if ((rs = stage(da, a, na, g.sms * 4, g.stream)) != GBNTT_OK) return rs;
         ua = da;
@@ -2561,9 +2566,8 @@ static int mul_host(uint32_t *c, const uint32_t *a, size_t na, const uint32_t *b
     const StageJob *stage_b = nullptr;
     if (square) ub = ua;
     else if (!ub) {
-        // B is copied by mul_dev on the copy stream (a small-grid copy
-        // kernel for pinned memory) after A's first pass: it then overlaps
-        // A's remaining passes instead of sharing the host link with them
+        // copied by mul_dev: by a kernel from pinned memory, on the copy
+        // stream with a small grid beside A's passes
         const uint32_t *mapped = g.zero_copy ? (const uint32_t *)pinned_device_ptr(b) : nullptr;
         jb.dst = db;
         jb.src = mapped ? mapped : b;

@@ -110,8 +110,8 @@ struct Residues<2> {
 // residues: 42.5 instead of 50.9 instructions per residue of a 2^8-point
 // pass. A forward 2^8-point pass over 6 2^25 residues takes 317 us instead of
 // 352, an inverse one over half of them 156 instead of 180 (FMA-heavy pipe
-// 68%, issue 0.61, DRAM 51%). It wants twice the tiles to fill the GPU
-// (launch_l).
+// 76 and 74%, issue 0.69 and 0.70, DRAM 61 and 60%). It wants twice the tiles
+// to fill the GPU (launch_l).
 template <int LOG_L, int DIR, bool LIMBS, int V>
 __global__ void __launch_bounds__(P31StridedShape<LOG_L, V, DIR, LIMBS>::T, P31StridedShape<LOG_L, V, DIR, LIMBS>::MIN_BLOCKS)
 p31_pass_kernel(const __grid_constant__ P31PassArgs a)

@@ -174,8 +174,9 @@ int gbntt_negacyclic_mul_u64(uint64_t *d_out, const uint64_t *d_f, const uint64_
  * product at a time): d_c[i][0 .. na[i]+nb[i]) = d_a[i] * d_b[i] for
  * i < count. The arrays are host arrays of device pointers and sizes. The
  * engine groups the products by transform length and runs each group in
- * waves that fit its workspace, one launch per pass and prime per wave.
- * Stream-ordered; results are bit-identical to gbntt_mul_u32 per product.
+ * waves that fit its workspace (products of more than 2^25 coefficients on
+ * the 31-bit primes one after the other). A batch that is refused computes no
+ * product. Stream-ordered; results are bit-identical to gbntt_mul_u32 per product.
  * Outputs must not overlap inputs or each other. */
 int gbntt_batch_mul_u32(uint32_t *const *d_c, const uint32_t *const *d_a, const size_t *na,
                         const uint32_t *const *d_b, const size_t *nb, int count, void *stream);
@@ -184,9 +185,9 @@ int gbntt_batch_mul_u32(uint32_t *const *d_c, const uint32_t *const *d_a, const 
  * server thread owning `slots` workspaces of 2^slot_log coefficients (48 x
  * 2^slot_log bytes of device memory each, on their own streams). Requests
  * are device-pointer products queued in arrival order; whenever a slot is
- * free the server admits, in arrival order, the pending requests of the
- * oldest request's transform length that fit the slot and runs them as one
- * wave, so requests arriving while others run are admitted as slots free
+ * free the server admits, in arrival order, the pending requests that fit
+ * the slot together, of any transform lengths, and runs them as one wave per
+ * length, so requests arriving while others run are admitted as slots free
  * up and their work overlaps on the device. Results are bit-identical to
  * gbntt_mul_u32. Latency = submit -> completion observed by the server.
  * The engine must be initialised; the ordinary entry points stay usable. */
@@ -362,8 +363,9 @@ int gbntt_compute_e(long digits, char *out, size_t cap, double *phase_seconds);
  * batches, serving, the e pipeline and ntt_bigint_mul in its default
  * mode): 2 = the fastest set for the length, the default: three 31-bit
  * primes (modulus ~2^92.6) for up to 2^29 coefficients with at most 2^28 limbs
- * in the shorter operand, else q0 = 2^64 - 2^32 + 1 (64-bit residues) with
- * p3 = 3 * 2^30 + 1 (32-bit residues), modulus ~2^95.6; 3 = the reference's
+ * in the shorter operand (served requests and cyclic products of the e
+ * pipeline: up to 3 * 2^25 points), else q0 = 2^64 - 2^32 + 1 (64-bit residues)
+ * with p3 = 3 * 2^30 + 1 (32-bit residues), modulus ~2^95.6; 3 = the reference's
  * three 64-bit primes (for packed and negacyclic products too). Products are
  * identical either way. The default comes from GBNTT_PRIMES (2 or 3) at
  * init; GBNTT_P31=0 leaves the 31-bit primes out. gbntt_prime_set returns 0
