@@ -15,9 +15,9 @@ Prints one JSON line. ``value`` is milliseconds per multiply with the
 operands already resident in HBM (CUDA events on the engine stream); ``e2e``
 is the same metric through the reference-facing C-ABI call ntt_bigint_mul on
 pinned host BigInts (2 GiB in, 2 GiB out per step, host wall clock).
-``--impl reference`` times the reference CPU path (the oracle restatement of
-the reference's scatter / NTT / Garner / gather, all host threads) on a
-bounded sample and scales it to the same metric.
+``cpu_baseline`` times the reference's CPU path (the oracle restatement of its
+scatter / NTT / Garner / gather, all host threads). The reference itself does
+not build for this GPU: ``--impl reference`` says so.
 
 Under torchrun (--gpus N > 1) every rank runs an independent replica on its
 own GPU (the multiply does not shard across GPUs); ``value`` is then the
@@ -53,7 +53,8 @@ def parse():
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--cpu-full", type=int, default=1,
                     help="also time one full-size product by the CPU port (all cores but one) and GMP (one core)")
-    ap.add_argument("--plan", default="", help="comma-separated pass sizes overriding the default plan")
+    ap.add_argument("--plan", default="", help="comma-separated pass sizes overriding the default plan of the full length (prime sets and "
+                         "lengths that run passes of it)")
     ap.add_argument("--no-packed", action="store_true", help="skip the packed (64-bit coefficient) measurement")
     ap.add_argument("--batch-pairs", type=int, default=4096)
     ap.add_argument("--batch-reps", type=int, default=2)
@@ -539,34 +540,10 @@ def run_e_leg(args):
 
 
 def run_reference(args, dist):
-    if dist.rank != 0:
-        return 0
-    times = []
-    res = None
-    for i in range(args.warmup + args.steps):
-        r = cpu_baseline(args.cpu_log_limbs, args.log_limbs, with_gmp=(i == args.warmup + args.steps - 1))
-        if i >= args.warmup:
-            times.append(r["value"])
-            res = r
-    v = float(np.median(times))
-    res["value"] = v
-    res["value_kind"] = "sample scaled by N log N"
-    if args.cpu_full and not args.no_cpu:
-        # one full-size product measured on the same cores: the scaled
-        # samples are reported next to it, with their error
-        full = cpu_full_size(args.log_limbs)
-        res["measured_full"] = full
-        if "port_s" in full:
-            res["measured_full_s"] = {"port": full["port_s"], "gmp_1thread": full.get("gmp_s")}
-            res["extrapolation_error"] = v / (full["port_s"] * 1e3) - 1.0
-    line = {"impl": "reference", "metric": METRIC, "value": v, "unit": UNIT, "n_gpus": args.gpus,
-            "steps": args.steps, "warmup": args.warmup, "ms_per_step": v, "higher_is_better": False,
-            "scaling": "weak", "vs_baseline": None, "dtype": "u64", "data": "synthetic (seeded splitmix64 limbs)",
-            "config": {"workload": "2^%d x 2^%d 32-bit limbs, N=2^%d, 3 primes" % (args.log_limbs, args.log_limbs,
-                                                                                    args.log_limbs + 1),
-                       "sample_log_limbs": args.cpu_log_limbs},
-            "cpu_baseline": res, "e2e": {"value": v, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-    print(json.dumps(line), flush=True)
+    if dist.rank == 0:
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "HIP and C for AMD GPUs, with no installable package and no NVIDIA build; its "
+                                         "CPU path, restated, is timed as cpu_baseline of the other arm"}), flush=True)
     return 0
 
 
@@ -838,7 +815,7 @@ def run_gpu(args, dist):
                              "modulus 2^92.6 > largest coefficient 2^92; the reference's three 64-bit primes "
                              "are timed in three_prime_64bit" if g.prime_set() == 2 else
                              "2^64-2^b+1, b = 32, 34, 40 (uint64 residues)",
-                   "operand_limbs": n, "transform_log": lg + 1, "passes": [log_l for kind, log_l, _, _ in recs if kind not in ("garner_carry", "carry")],
+                   "operand_limbs": n, "transform_log": lg + 1, "passes": [log_l for kind, log_l, _, _ in recs if "pass" in kind],
                    "l2_policy": "inputs and 12 GiB spectra >> 129 MB L2; no flush", "parallelism": "replicas"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "peak_source": peak_kind,
