@@ -54,6 +54,24 @@ struct ShoupWord {
 };
 constexpr ShoupWord shoup_word(uint64_t w, uint64_t p) { return {(uint32_t)w, (uint32_t)((w << 32) / p)}; }
 
+// t[i] = w^i in Montgomery form, i < n: each length's powers from the first
+// half's times one factor (Shoup).
+static inline void p31_powers(uint32_t *t, size_t n, uint64_t w, uint64_t p)
+{
+    const uint32_t q = (uint32_t)p;
+    t[0] = (uint32_t)(((uint64_t)1 << 32) % p);
+    for (size_t m = 1; m < n; m *= 2, w = w * w % p) {
+        const ShoupWord f = shoup_word(w, p);   // w^m
+        const uint32_t *__restrict__ a = t;
+        uint32_t *__restrict__ b = t + m;
+        const size_t end = n - m < m ? n - m : m;
+        for (size_t i = 0; i < end; i++) {
+            const uint32_t r = a[i] * f.w - (uint32_t)(((uint64_t)a[i] * f.q) >> 32) * q, s = r - q;
+            b[i] = s < r ? s : r;   // (r < 2 p)
+        }
+    }
+}
+
 // w_32^i per prime and direction: the constants of the register DFTs.
 struct P31Roots {
     ShoupWord v[3][2][16];
@@ -390,6 +408,18 @@ cudaError_t launch_p31_nega_finish(const P31NegaArgs &a, cudaStream_t st);
 cudaError_t launch_p31_pass(int log_l, int dir, bool limbs, int nops, const P31PassArgs &a, cudaStream_t st);
 cudaError_t launch_p31_contig_fwd(int log_l, const P31InnerArgs &a, cudaStream_t st);
 cudaError_t launch_p31_inner(int log_l, const P31InnerArgs &a, cudaStream_t st);
+// Powers of w in Montgomery form on the device: t[i] = w^i, i < n, prime k
+// (w: 2^32 times the root).
+constexpr int kP31MaxPowers = 48;
+struct P31PowersArgs {
+    struct {
+        uint32_t *t;
+        uint32_t n, w;
+        int k;
+    } job[kP31MaxPowers];
+    int njobs;
+};
+cudaError_t launch_p31_powers(const P31PowersArgs &a, cudaStream_t st);
 cudaError_t launch_p31_build_table(int prime, uint32_t *table, const uint32_t *hi, const uint32_t *lo, int log_m,
                                    int log_s, int use_scale, uint32_t scale, cudaStream_t st);
 

@@ -351,12 +351,7 @@ int fill_tables(uint32_t *dst, uint64_t w, uint64_t p)   // w of order N; return
         const int lm = S::log_m(s), ls = lm - S::log_r(s);
         const uint64_t wm = p31_pow(w, 1ull << (LOG_N - lm), p);
         for (int k = 0; k < 1 << S::log_r(s); k++) {
-            const uint64_t wk = p31_pow(wm, (uint64_t)k, p);
-            uint64_t x = 1;
-            for (int j = 0; j < 1 << ls; j++) {
-                dst[off + (k << ls) + j] = (uint32_t)((x << 32) % p);
-                x = x * wk % p;
-            }
+            p31_powers(dst + off + (k << ls), (size_t)1 << ls, p31_pow(wm, (uint64_t)k, p), p);
         }
         off += 1 << lm;
     }

@@ -288,13 +288,15 @@ cudaError_t p31_outer_init()
             std::vector<uint64_t> c(n);
             for (int m = 0; m < n; m++) c[m] = p31_pow(gamma, (uint64_t)m * (paired ? 2 : 1), p);
             const std::vector<uint64_t> v = vandermonde_inverse(c, p);
-            for (int r = 0; r < n; r++)
-                for (int m = 0; m < n; m++) {
+            for (int m = 0; m < n; m++) {
+                const uint64_t odd = p31_pow(p31_pow(gamma, (uint64_t)m, p), p - 2, p);
+                for (int r = 0; r < n; r++) {
                     const uint64_t x = v[(size_t)r * n + m], half = x * ((p + 1) / 2) % p;
                     dst[r * kMaxR + m] = mont(paired ? half : x);
                     if (paired)   // the differences are 2 gamma^m times the odd blocks' polynomial
-                        dst[r * kMaxR + kMaxR / 2 + m] = mont(half * p31_pow(p31_pow(gamma, (uint64_t)m, p), p - 2, p) % p);
+                        dst[r * kMaxR + kMaxR / 2 + m] = mont(half * odd % p);
                 }
+            }
         }
     return cudaMemcpyToSymbol(c_inv, h.data(), h.size() * sizeof(uint32_t));
 }

@@ -458,6 +458,21 @@ cudaError_t launch_l(int dir, bool limbs, int nops, P31PassArgs &a, cudaStream_t
     return launch_v<LOG_L, 1>(dir, limbs, nops, a, st);
 }
 
+__global__ void p31_powers_kernel(const __grid_constant__ P31PowersArgs a)
+{
+    const auto &j = a.job[blockIdx.y];
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= j.n) return;
+    const uint32_t p = p31_prime(j.k), pinv = p31_inv(j.k);
+    uint32_t x = 0u - 2u * p < p ? 0u - 2u * p : 0u - 3u * p;   // 2^32 mod p, 2 p < 2^32 < 4 p
+    uint32_t b = j.w;
+    for (uint32_t e = i; e; e >>= 1) {
+        if (e & 1) x = p31_mont(x, b, p, pinv);
+        b = p31_mont(b, b, p, pinv);
+    }
+    j.t[i] = x;
+}
+
 __global__ void p31_table_kernel(int k, uint32_t *table, const uint32_t *hi, const uint32_t *lo, int log_m, int log_s,
                                  int use_scale, uint32_t scale)
 {
@@ -487,6 +502,15 @@ cudaError_t launch_p31_pass(int log_l, int dir, bool limbs, int nops, const P31P
     case 10: return launch_l<10>(dir, limbs, nops, a, st);
     default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t launch_p31_powers(const P31PowersArgs &a, cudaStream_t st)
+{
+    uint32_t n = 0;
+    for (int i = 0; i < a.njobs; i++) n = n > a.job[i].n ? n : a.job[i].n;
+    if (a.njobs < 1 || a.njobs > kP31MaxPowers || n == 0) return cudaErrorInvalidValue;
+    p31_powers_kernel<<<dim3((n + 255) / 256, (unsigned)a.njobs), 256, 0, st>>>(a);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_p31_build_table(int prime, uint32_t *table, const uint32_t *hi, const uint32_t *lo, int log_m,
